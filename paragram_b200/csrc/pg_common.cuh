@@ -40,6 +40,18 @@ constexpr int kMaxWarpsPerSM = 32;  // upper bound of resident cell warps per SM
 constexpr int kBigWarps = 4;        // warps per block of the 256-slot tier (state in shared memory)
 constexpr int kMidWarps = 4;        // warps per block of the 128-slot tier (13 KB of shared memory each)
 constexpr int kMidBlocksPerSM = 3;  // its resident blocks per SM (up to 170 registers per thread)
+#ifndef PG_LANE_V
+#define PG_LANE_V 48
+#endif
+#ifndef PG_LANE_WARM
+#define PG_LANE_WARM 16
+#endif
+#ifndef PG_LANE_MIN
+#define PG_LANE_MIN 32768
+#endif
+constexpr int kLaneV = PG_LANE_V;       // vertex slots of a cell of the cell-per-lane pass
+constexpr int kLaneWarm = PG_LANE_WARM; // nearest points that clip it first
+constexpr int64_t kLaneMinCells = PG_LANE_MIN; // smallest build of that pass
 constexpr int kMaxLeaf = 32;        // leaf size limit (one candidate per lane)
 constexpr int kDefaultLeaf = 16;
 constexpr int kWindow = 16;         // optional warm start: sorted neighbours i-16 .. i+16

@@ -37,10 +37,10 @@
 
 #if defined(__CUDACC__)
 #define PG_HD __host__ __device__ __forceinline__
-#define PG_HD_NOINLINE __host__ __device__ __noinline__
+#define PG_HD_NOINLINE static __host__ __device__ __noinline__
 #else
 #define PG_HD inline
-#define PG_HD_NOINLINE
+#define PG_HD_NOINLINE static
 #endif
 
 namespace pg

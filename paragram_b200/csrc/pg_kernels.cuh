@@ -44,9 +44,19 @@ struct CellLaunch
     int *vertex_count_out;     // per original id: number of vertices
     int use_hint;      // the workspace holds a search radius per sorted slot
     int fp32_only;     // side tests in FP32 only (no escalation; not exact)
+    int lanes;         // one cell per lane (pg_lane.cu), then cells_list_launch for those that do not fit
 };
+void cells_list_launch(const Workspace &ws, const CellLaunch &cl, int *status, int num_sms, cudaStream_t st);
 void cells_launch(const Workspace &ws, const CellLaunch &cl, int *status, int num_sms, cudaStream_t st);
 void cells_big_launch(const Workspace &ws, const CellLaunch &cl, int *status, int64_t big_cap, cudaStream_t st);
+
+// pg_lane.cu
+struct CellArgs;
+void lane_launch(const CellArgs &A, int *list, int num_sms, cudaStream_t st);
+
+// pg_knn.cu: the kLaneWarm nearest other points (sorted slots, nearest first, -1: none) of the
+// sorted slots [begin, end), into the cells' rows
+void knn_rows_launch(const Workspace &ws, int num_clouds, int64_t begin, int64_t end, cudaStream_t st);
 
 // pg_mlp.cu
 void features_launch(const Workspace &ws, int64_t n, int num_clouds, float *out, cudaStream_t st);

@@ -1,0 +1,387 @@
+// pg_lane.cu -- per-cell convex clipping, one cell per lane.
+//
+// The first pass of builds that fill the GPU (build_impl's rule). The same clipping
+// and the same exact predicates as pg_cells.cu (reference counterpart:
+// voronoi_ultra.cu:39-141, laguerre_ultra.cu:43-174, also one thread per cell), so
+// the cells are the same; what differs is who does the work. A warp per cell issues
+// every step of a cell's search once per cell (28,900 warp instructions for a cell of
+// about 27 vertices, 21.8 of 32 lanes active); 32 cells per warp, kept in step, share
+// them: 8,100 for 32 cells' steps per cell.
+//
+// What keeps the lanes in step: (1) a cell is first clipped by its kLaneWarm nearest
+// points (k_knn_rows), nearly all of which cut it; (2) the points that can still
+// reach it come from one search of the BVH for the warp's 32 cells, whose nodes and
+// leaves every lane tests at the same time; (3) the points in reach are tested four
+// at a time against the vertices, and only those that may cut (about 8 of 50) are
+// kept for clipping; (4) in clipping every lane first looks for its next point that
+// cuts, then all clip. Lanes that search on their own (a traversal per lane, whether
+// left to diverge or scheduled step by step) ran at 4 to 10 active lanes: 45 and
+// 22 ms for 500,000 clustered cells, against 21 ms for a warp per cell and 12 here.
+// Eight lanes per cell: 26 ms (instruction-cache misses between the steps).
+//
+// A cell that does not fit (more than kLaneV vertices or kLaneP planes at a time, a
+// reach that holds more than kLaneMarks points: cells at the hull, beside a far denser
+// region, or long cells of surface data) is listed for the warp-per-cell pass.
+//
+// Measured on one B200, first pass with its kNN query and listed cells: 5M clustered
+// points 214 -> 103 ms, 1M uniform power 43.6 -> 21.4 ms, jittered 128^3 power lattice
+// 87.5 -> 21.9 ms. Bound by latency: one warp per block, 7 blocks per SM (31 KB of shared
+// memory each), 33% of the issue slots used.
+#include <algorithm>
+
+#include "pg_kernels.cuh"
+#include "pg_lane.cuh"
+
+namespace pg
+{
+
+#ifndef PG_LANE_BLOCKS
+#define PG_LANE_BLOCKS 7
+#endif
+#ifndef PG_LANE_SHELL
+#define PG_LANE_SHELL 2.5f
+#endif
+#ifndef PG_LANE_FAR
+#define PG_LANE_FAR 6.0f
+#endif
+#ifndef PG_LANE_MARKS
+#define PG_LANE_MARKS 96
+#endif
+constexpr int kLaneBlocks = PG_LANE_BLOCKS; // resident one-warp blocks per SM (31 KB of shared memory each)
+// Squared radius of the first search over the last near point's. 500,000 clustered cells: 2.0 14.5, 2.5 13.8,
+// 3.0 14.8 ms (a smaller one leaves more cells to the second search, a larger one more points to test).
+constexpr float kLaneShell = PG_LANE_SHELL;
+constexpr float kLaneFar = PG_LANE_FAR;     // the largest that a cell may need after it (beyond: listed)
+constexpr int kLaneTrial = 128;             // warps' worth of cells before their outcome decides about the rest
+constexpr int kLaneMarks = PG_LANE_MARKS;   // points of a search within a cell's reach
+
+// Optional per-phase SM cycle counters, as in pg_cells.cu (compile with -DPG_PHASE_CYCLES): the clips by the
+// nearest points, the search, its tests, the clips by its points, and whole cells, per cell.
+#ifdef PG_PHASE_CYCLES
+#define PG_LANE_T0(t) long long t = clock64()
+#define PG_LANE_T1(cell, k, t)                                                                                         \
+    do                                                                                                                 \
+    {                                                                                                                  \
+        const long long pg_now_ = clock64();                                                                           \
+        (cell).cyc[k] += pg_now_ - (t);                                                                                \
+        (t) = pg_now_;                                                                                                 \
+    } while (0)
+#else
+#define PG_LANE_T0(t)
+#define PG_LANE_T1(cell, k, t)
+#endif
+
+__device__ __forceinline__ float lane_box_dist(float4 s, float lx, float ly, float lz, float hx, float hy, float hz)
+{
+    const float dx = fmaxf(fmaxf(lx - s.x, s.x - hx), 0.0f), dy = fmaxf(fmaxf(ly - s.y, s.y - hy), 0.0f),
+                dz = fmaxf(fmaxf(lz - s.z, s.z - hz), 0.0f);
+    return (dx * dx + dy * dy + dz * dz) * (1.0f - 1e-5f);
+}
+
+// 32 consecutive cells of the curve order per warp at a time (persistent warps, cells from a counter).
+__global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int *list)
+{
+    __shared__ LaneMem m;
+    const int lane = threadIdx.x;
+    LaneCell C(m, A, lane);
+    unsigned cmask[kLaneLeaves / 2];
+    int cand[kLaneCut];
+    for (;;)
+    {
+        int g = 0;
+        if (lane == 0)
+            g = atomicAdd(&A.counters[0], 1);
+        g = __shfl_sync(kFull, g, 0);
+        const int64_t gb = A.begin + (int64_t)g * 32;
+        if (gb >= A.end)
+            break;
+        const bool act = gb + lane < A.end;
+        {
+            // Where most cells so far had to be listed (surface data: long cells whose reach holds far too many
+            // points), the rest is listed at once. A cell costs 18 ns here against 45 to 70 ns in the
+            // warp-per-cell pass, so two in three have to succeed to pay for the rest.
+            int at = -1;
+            if (lane == 0)
+            {
+                const int done = __ldcg(&A.counters[9]), listed = __ldcg(&A.counters[8]);
+                if (done >= kLaneTrial && listed > done * 20)
+                    at = atomicAdd(&A.counters[8], (int)min((int64_t)32, A.end - gb));
+            }
+            at = __shfl_sync(kFull, at, 0);
+            if (at >= 0)
+            {
+                if (act)
+                {
+                    const int i = (int)gb + lane, u = A.oid[i];
+                    A.deg[u] = 0;
+                    A.status[u] = kPlaneOverflow; // placeholder until the pass over the list
+                    list[at + lane] = i;
+                }
+                continue;
+            }
+        }
+        C.init((int)(act ? gb + lane : A.end - 1));
+        C.alive = C.alive && act;
+        PG_LANE_T0(t0);
+        // Its nearest points (sorted slots, nearest first, -1: none, left in the cell's row) clip a cell first,
+        // then the other points within reach, in up to three shells around it. No point farther than
+        // R + sqrt(R^2 + w) can cut a cell of radius R, w the excess of the cloud's largest weight over the
+        // seed's: its bisector distance (d^2 - dw) / (2 d) exceeds R.
+        int nk = 0, jK = -1;
+        {
+            const int4 *kn = reinterpret_cast<const int4 *>(A.rows + (size_t)C.soid * kRowWidth);
+#pragma unroll
+            for (int t = 0; t < kLaneWarm / 4; ++t)
+            {
+                const int4 k4 = kn[t];
+                cand[4 * t + 0] = k4.x;
+                cand[4 * t + 1] = k4.y;
+                cand[4 * t + 2] = k4.z;
+                cand[4 * t + 3] = k4.w;
+                nk += (k4.x >= 0) + (k4.y >= 0) + (k4.z >= 0) + (k4.w >= 0);
+                jK = k4.w;
+            }
+            if (C.alive && jK == -2)
+                C.give_up();
+            if (!C.alive)
+                nk = 0;
+        }
+        bool search = C.alive && jK >= 0; // (fewer points than that: all of them are in the list)
+        const float dK = search ? lane_sq_dist(C.s, A.pts[jK]) : 0.0f;
+        if (!(dK < 1e30f))
+        {
+            C.give_up(); // out of the squared distances' range
+            nk = 0;
+            search = false;
+        }
+        const float dwm = search ? fmaxf(C.box[6] - C.s.w, 0.0f) * (1.0f + 1e-6f) : 0.0f;
+        float lo = dK, hi = 0.0f;
+#pragma unroll 1
+        for (int shell = -1; shell < 3; ++shell)
+        {
+            if (shell >= 0)
+            {
+                search = search && C.alive;
+                if (search)
+                {
+                    C.radius();
+                    float need = C.rsafe + sqrtf(fmaf(C.rsafe, C.rsafe, dwm));
+                    need = need * need * (1.0f + 4e-5f);
+                    if (need <= lo)
+                        search = false; // every point within reach was clipped
+                    else if (shell == 2 || (shell == 1 && need > kLaneFar * dK))
+                    {
+                        C.give_up();
+                        search = false;
+                    }
+                    hi = shell == 0 ? fminf(need, kLaneShell * dK) : need;
+                }
+                if (!__any_sync(kFull, search))
+                    break;
+                // Points with lo <= d^2 <= hi of every lane's cell: one search of the BVH for the warp's 32 cells.
+                // Leaves within reach of some lane are listed, scanned in pairs into a bit mask per lane, and the
+                // marked points tested; those that may remove a vertex of the present cell are kept.
+                nk = 0;
+                int sp = 0, marks = 0;
+                bool over = false;
+                float rr = -1.0f;
+                for (unsigned todo = __ballot_sync(kFull, search);;)
+                {
+                    if (sp == 0)
+                    {
+                        if (todo == 0u || over)
+                            break;
+                        // (a warp's cells may belong to several clouds)
+                        const int root = __shfl_sync(kFull, C.root, __ffs(todo) - 1);
+                        const bool mine = search && C.root == root;
+                        todo &= ~__ballot_sync(kFull, mine);
+                        rr = mine ? hi : -1.0f;
+                        if (lane == 0)
+                            m.stk[0] = root;
+                        sp = 1;
+                        __syncwarp();
+                    }
+                    int nl = 0;
+                    while (sp > 0 && nl <= kLaneLeaves - 4)
+                    {
+                        // two nodes at a time: their loads overlap
+                        const int two = sp > 1 ? 1 : 0;
+                        const float4 *pa = A.rec + 4 * (size_t)m.stk[sp - 1], *pb = A.rec + 4 * (size_t)m.stk[sp - 1 - two];
+                        const float4 a0 = pa[0], a1 = pa[1], a2 = pa[2], a3 = pa[3];
+                        const float4 b0 = pb[0], b1 = pb[1], b2 = pb[2], b3 = pb[3];
+                        sp -= 1 + two;
+                        const bool h0 = __any_sync(kFull, lane_box_dist(C.s, a0.x, a0.y, a0.z, a0.w, a1.x, a1.y) <= rr);
+                        const bool h1 = __any_sync(kFull, lane_box_dist(C.s, a1.z, a1.w, a2.x, a2.y, a2.z, a2.w) <= rr);
+                        const bool h2 =
+                            two && __any_sync(kFull, lane_box_dist(C.s, b0.x, b0.y, b0.z, b0.w, b1.x, b1.y) <= rr);
+                        const bool h3 =
+                            two && __any_sync(kFull, lane_box_dist(C.s, b1.z, b1.w, b2.x, b2.y, b2.z, b2.w) <= rr);
+                        C.n_nodes += rr >= 0.0f ? 2u + 2u * two : 0u;
+                        if (sp + 4 > kLaneStack)
+                        {
+                            over = true;
+                            sp = 0;
+                            break;
+                        }
+                        const bool h[4] = {h0, h1, h2, h3};
+                        const float f4[4] = {a3.x, a3.y, b3.x, b3.y};
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+                            if (h[c])
+                            {
+                                const int f = __float_as_int(f4[c]);
+                                if (lane == 0)
+                                    (f < 0 ? m.lv[nl] : m.stk[sp]) = f;
+                                nl += f < 0 ? 1 : 0;
+                                sp += f < 0 ? 0 : 1;
+                            }
+                        __syncwarp();
+                    }
+                    if (over)
+                        break;
+                    C.n_leaves += rr >= 0.0f ? nl : 0;
+                    if (lane == 0)
+                        m.lv[nl] = 0; // the last pair may have one leaf
+                    __syncwarp();
+                    const int nr = (nl + 1) >> 1;
+                    auto load = [&](int k) -> float4 {
+                        const int ref = m.lv[2 * k + (lane >> 4)];
+                        return ref < 0 && (lane & 15) < leaf_count(ref) ? A.pts[leaf_first(ref) + (lane & 15)]
+                                                                        : make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
+                    };
+                    float4 pt = load(0);
+                    for (int k = 0; k < nr; ++k)
+                    {
+                        m.pt[lane] = pt;
+                        __syncwarp();
+                        if (k + 1 < nr)
+                            pt = load(k + 1);
+                        unsigned mask = 0;
+#pragma unroll
+                        for (int p = 0; p < 32; ++p)
+                        {
+                            const float d = lane_sq_dist(C.s, m.pt[p]);
+                            if (d >= lo && d <= rr)
+                                mask |= 1u << p;
+                        }
+                        cmask[k] = mask;
+                        marks += __popc(mask);
+                        if (marks > kLaneMarks)
+                        {
+                            // a far denser region within reach: listed, and no longer part of the search
+                            C.give_up();
+                            rr = -1.0f;
+                            marks = INT_MIN;
+                        }
+                        __syncwarp();
+                    }
+                    PG_LANE_T1(C, kLaneCycSearch, t0);
+                    // all lanes test up to four of their points at a time
+                    int rd = rr >= 0.0f ? 0 : nr;
+                    unsigned mw = 0;
+                    for (;;)
+                    {
+                        int j[4];
+                        Cand cq[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                        {
+                            while (mw == 0u && rd < nr)
+                                mw = cmask[rd++];
+                            j[u] = -1;
+                            if (mw != 0u)
+                            {
+                                const int b = __ffs(mw) - 1;
+                                mw &= mw - 1u;
+                                j[u] = leaf_first(m.lv[2 * (rd - 1) + (b >> 4)]) + (b & 15);
+                            }
+                        }
+                        if (!__any_sync(kFull, j[0] >= 0))
+                            break;
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            cq[u] = make_cand(C.s, A.pts[max(j[u], 0)], j[u]);
+                        const unsigned may = j[0] >= 0 ? C.may_cut4(cq) : 0u;
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (j[u] >= 0 && ((may >> u) & 1u) &&
+                                !(shell == 0 && j[u] <= jK && lane_sq_dist(C.s, A.pts[j[u]]) == dK)) // (clipped before)
+                            {
+                                if (nk < kLaneCut)
+                                    cand[nk] = j[u];
+                                ++nk;
+                            }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            C.n_cands += j[u] >= 0 ? 1u : 0u;
+                        __syncwarp();
+                    }
+                    PG_LANE_T1(C, kLaneCycTests, t0);
+                }
+                if ((over && search) || nk > kLaneCut)
+                {
+                    C.give_up();
+                }
+                if (!C.alive)
+                    nk = 0;
+                lo = __uint_as_float(__float_as_uint(hi) + 1u); // the next shell begins beyond hi
+            }
+            __syncwarp();
+            PG_LANE_T1(C, kLaneCycTests, t0);
+            // clip by the listed points that cut: every lane looks for its next one, then all clip
+            int jn = nk > 0 ? cand[0] : 0;
+            float4 qn = A.pts[jn];
+            for (int c = 0;;)
+            {
+                bool cut = false;
+                unsigned r0 = 0, r1 = 0;
+                Cand cq;
+                int j = -1;
+                while (c < nk && !cut)
+                {
+                    j = jn;
+                    const float4 q = qn;
+                    if (++c < nk) // (loaded beside this point's tests)
+                    {
+                        jn = cand[c];
+                        qn = A.pts[jn];
+                    }
+                    if (q.x == C.s.x && q.y == C.s.y && q.z == C.s.z)
+                        continue; // coincident points do not clip each other
+                    cq = make_cand(C.s, q, j);
+                    cut = C.classify(cq, j, r0, r1);
+                    if (!C.alive)
+                        nk = 0;
+                }
+                __syncwarp();
+                if (__ballot_sync(kFull, cut) == 0u)
+                    break;
+                if (cut)
+                {
+                    C.update(cq, j, r0, r1);
+                    if (!C.alive)
+                        nk = 0;
+                }
+                __syncwarp();
+                PG_LANE_T1(C, shell < 0 ? kLaneCycNear : kLaneCycClips, t0);
+            }
+        }
+        __syncwarp();
+        if (act)
+            C.output(list, &A.counters[8]);
+        __syncwarp();
+        if (lane == 0)
+            atomicAdd(&A.counters[9], 1);
+    }
+    C.flush();
+}
+
+void lane_launch(const CellArgs &A, int *list, int num_sms, cudaStream_t st)
+{
+    const int64_t need = (A.end - A.begin + 31) / 32;
+    const int64_t grid = std::min<int64_t>((int64_t)num_sms * kLaneBlocks, need);
+    ++g_launches;
+    k_cells_lane<<<(unsigned)std::max<int64_t>(grid, 1), 32, 0, st>>>(A, list);
+}
+
+} // namespace pg

@@ -1,0 +1,87 @@
+"""The cell-per-lane first pass (builds of at least kLaneMinCells cells, pg_lane.cu) against the oracle, at
+the sizes and inputs where its rules end: the last warp's idle lanes, coincident
+points, cells of more than 48 vertices, reaches that hold too many points, chunks."""
+
+import numpy as np
+import pytest
+import torch
+
+from _helpers import diff_cells
+
+pytestmark = pytest.mark.gpu
+
+MIN = 32768  # kLaneMinCells
+
+
+@pytest.fixture(scope="module")
+def dev():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    return torch.device("cuda:0")
+
+
+def _cloud(kind, n, seed=5):
+    from paragram_b200 import workloads as W
+
+    rng = np.random.default_rng(seed)
+    w = None
+    if kind == "uniform":
+        p = W.uniform(n, seed)
+    elif kind == "power":
+        p, w = W.power_uniform(n, seed)
+    elif kind == "heavy":  # weights that empty many cells and move others off their points
+        p = W.uniform(n, seed)
+        w = (rng.random(n) * 4.0 * n ** (-2.0 / 3.0)).astype(np.float32)
+    elif kind == "lattice":
+        m = round(n ** (1 / 3))
+        p, w = W.jittered_lattice(m, seed)
+    elif kind == "exact_lattice":
+        m = round(n ** (1 / 3))
+        g = np.arange(m, dtype=np.float32) / np.float32(64.0)
+        p = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3).copy()
+    elif kind == "surface":
+        p = W.surface_cloud(n, np.random.Generator(np.random.PCG64(seed)))
+    elif kind == "dense_spots":  # a tenth of the points in 40 spots a thousandth of the spacing wide
+        p = W.uniform(n, seed)
+        k = n // 10
+        p[:k] = p[k:k + 40][rng.integers(0, 40, k)] + (1e-5 * rng.standard_normal((k, 3))).astype(np.float32)
+    elif kind == "coincident":  # every fourth point is a copy, some places hold twenty
+        p = W.uniform(n, seed)
+        p[::4] = p[1::4][: len(p[::4])]
+        p[:200] = np.repeat(p[300:310], 20, axis=0)
+    elif kind == "wheel":  # hubs with 60 points around each: cells beyond 48 vertices
+        hubs = W.uniform(n // 61, seed)
+        a = rng.random((len(hubs), 60)) * 2 * np.pi
+        d = 0.3 * len(hubs) ** (-1.0 / 3.0)
+        ring = hubs[:, None, :] + d * np.stack([np.cos(a), np.sin(a), 0.05 * rng.standard_normal(a.shape)], -1)
+        p = np.concatenate([hubs, ring.reshape(-1, 3)]).astype(np.float32)
+    return np.ascontiguousarray(p), w
+
+
+def _gpu(p, w, dev, **kw):
+    import paragram_b200.cuda as pc
+
+    t = torch.from_numpy(p).to(dev)
+    tw = None if w is None else torch.from_numpy(w).to(dev)
+    (a, o, s), st = pc.build_with_stats(t, tw, **kw)
+    return (a.cpu().numpy(), o.cpu().numpy(), s.cpu().numpy()), st
+
+
+@pytest.mark.parametrize("kind,n", [("uniform", MIN - 1), ("uniform", MIN), ("uniform", MIN + 1), ("power", MIN + 31),
+                                    ("heavy", 40_000), ("lattice", 35_937), ("exact_lattice", 35_937),
+                                    ("surface", 36_001), ("dense_spots", 40_000), ("coincident", 36_000),
+                                    ("wheel", 36_600)])
+def test_lane_pass_equals_oracle(dev, oracle, kind, n):
+    p, w = _cloud(kind, n)
+    got, _ = _gpu(p, w, dev)
+    assert diff_cells(got, oracle.diagram(p, w)).size == 0
+
+
+def test_lane_pass_equals_warp_pass_and_chunks(dev):
+    """blocks_per_sm = 2 keeps the warp-per-cell pass; chunks split the lane pass's launches."""
+    p, w = _cloud("power", 50_001)
+    ref, _ = _gpu(p, w, dev, blocks_per_sm=2)
+    for chunks in (1, 3, 7):
+        got, st = _gpu(p, w, dev, num_chunks=chunks)
+        assert all(np.array_equal(x, y) for x, y in zip(got, ref)), chunks
+        assert st["clips"] > 10 * len(p)
