@@ -424,15 +424,14 @@ static int build_impl(int64_t n, int num_clouds, const int32_t *cloud_offsets, c
         k_hint_gather<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, ws.oid, opt.radius_hint, ws.hint);
         cl.use_hint = 1;
     }
-    // One cell per lane (pg_lane.cu) where that fills the GPU and nothing but the diagram is asked for: a lane
+    // One cell per lane (pg_lane.cu) where that fills the GPU and no per-cell diagnostics are asked for: a lane
     // takes about 0.9 ms for its cell however few there are, so below kLaneMinCells the warp-per-cell pass is
     // faster (uniform points: 24,000 1.60 against 1.61 ms, 32,000 2.22 against 1.98, 96,000 5.19 against 3.51;
     // clustered: 48,000 3.17 against 3.34, 64,000 3.80 against 3.60). Its leaf scans take leaves of up to 16
     // points. Batches are mostly surface clouds, whose cells it leaves to the warp-per-cell pass.
     const int64_t cells = ranged ? range_end - range_begin : n;
-    cl.lanes = cells >= kLaneMinCells && num_clouds == 1 && leaf <= kDefaultLeaf && !guesses && !cl.use_hint &&
-               !cl.fp32_only && !opt.radius_out && !opt.work_out && !opt.geometry_out && !opt.vertices_out &&
-               !opt.vertex_planes_out && !opt.vertex_count_out && opt.blocks_per_sm == 0;
+    cl.lanes = cells >= kLaneMinCells && num_clouds == 1 && leaf <= kDefaultLeaf && !cl.fp32_only &&
+               !opt.radius_out && !opt.work_out && opt.blocks_per_sm == 0;
     int chunks = sync ? plan_chunks(n, opt.num_chunks) : std::max(opt.num_chunks, 1);
     int sms = device_sms();
     const int64_t rb = ranged ? range_begin : 0, re = ranged ? range_end : n;

@@ -79,6 +79,10 @@ __device__ __forceinline__ float lane_box_dist(float4 s, float lx, float ly, flo
 }
 
 // 32 consecutive cells of the curve order per warp at a time (persistent warps, cells from a counter).
+// GUESS: the caller's initial guesses clip a cell first, in the place of its nearest points. EXPORT: geometry
+// and vertices are asked for. A search radius per cell (A.hint: learned or given) bounds its first search; a
+// negative one marks a cell that the model routed past this pass.
+template <bool GUESS, bool EXPORT>
 __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int *list)
 {
     __shared__ LaneMem m;
@@ -95,7 +99,7 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
         const int64_t gb = A.begin + (int64_t)g * 32;
         if (gb >= A.end)
             break;
-        const bool act = gb + lane < A.end;
+        bool act = gb + lane < A.end;
         {
             // Where most cells so far had to be listed (surface data: long cells whose reach holds far too many
             // points), the rest is listed at once. A cell costs 18 ns here against 45 to 70 ns in the
@@ -104,7 +108,7 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
             if (lane == 0)
             {
                 const int done = __ldcg(&A.counters[9]), listed = __ldcg(&A.counters[8]);
-                if (done >= kLaneTrial && listed > done * 20)
+                if (done >= kLaneTrial && listed > done * 20 && A.hint == nullptr)
                     at = atomicAdd(&A.counters[8], (int)min((int64_t)32, A.end - gb));
             }
             at = __shfl_sync(kFull, at, 0);
@@ -121,13 +125,45 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
             }
         }
         C.init((int)(act ? gb + lane : A.end - 1));
+        float hint = INFINITY; // search radius
+        if (A.hint != nullptr)
+        {
+            const float r = A.hint[C.i];
+            if (r > 0.0f && r < 1e30f)
+                hint = r;
+            act = act && !(r < 0.0f);
+        }
         C.alive = C.alive && act;
         PG_LANE_T0(t0);
         // Its nearest points (sorted slots, nearest first, -1: none, left in the cell's row) clip a cell first,
-        // then the other points within reach, in up to three shells around it. No point farther than
+        // then the other points within reach, in shells around it. No point farther than
         // R + sqrt(R^2 + w) can cut a cell of radius R, w the excess of the cloud's largest weight over the
         // seed's: its bisector distance (d^2 - dw) / (2 d) exceeds R.
         int nk = 0, jK = -1;
+        float dK = 0.0f; // squared distance of the last of them, the scale of the search
+        bool search = C.alive;
+        if (GUESS)
+        {
+            const int g0 = A.guess_off[C.soid], g1 = A.guess_off[C.soid + 1];
+            if (C.alive && g1 - g0 > kLaneCut)
+                C.give_up();
+            for (int k = g0; C.alive && k < g1; ++k)
+            {
+                const int o = A.guesses[k];
+                const int j = o >= 0 && o < A.n ? A.rank[o] : -1;
+                // (a guess in another cloud is a point all the same)
+                if (j >= 0 && j != C.i)
+                {
+                    cand[nk++] = j;
+                    dK += __log2f(fmaxf(lane_sq_dist(C.s, A.pts[j]), 1e-30f));
+                }
+            }
+            // the scale of the search: the geometric mean, which the far neighbours of a cell at the hull hardly
+            // move, to about where the 16th nearest point lies (1.6 times it among uniform points)
+            dK = nk > 0 ? 1.6f * exp2f(dK / (float)nk) : 0.0f;
+            search = C.alive;
+        }
+        else
         {
             const int4 *kn = reinterpret_cast<const int4 *>(A.rows + (size_t)C.soid * kRowWidth);
 #pragma unroll
@@ -143,21 +179,21 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
             }
             if (C.alive && jK == -2)
                 C.give_up();
-            if (!C.alive)
-                nk = 0;
+            search = C.alive && jK >= 0; // (fewer points than that: all of them are in the list)
+            if (search)
+                dK = lane_sq_dist(C.s, A.pts[jK]);
         }
-        bool search = C.alive && jK >= 0; // (fewer points than that: all of them are in the list)
-        const float dK = search ? lane_sq_dist(C.s, A.pts[jK]) : 0.0f;
-        if (!(dK < 1e30f))
+        if (search && !(dK > 0.0f && dK < 1e30f))
         {
-            C.give_up(); // out of the squared distances' range
-            nk = 0;
+            C.give_up(); // no scale to search by: no guesses, or coincident points only
             search = false;
         }
+        if (!C.alive)
+            nk = 0;
         const float dwm = search ? fmaxf(C.box[6] - C.s.w, 0.0f) * (1.0f + 1e-6f) : 0.0f;
-        float lo = dK, hi = 0.0f;
+        float lo = GUESS ? 0.0f : dK, hi = 0.0f; // the points nearer than lo were clipped
 #pragma unroll 1
-        for (int shell = -1; shell < 3; ++shell)
+        for (int shell = -1; shell < 4; ++shell)
         {
             if (shell >= 0)
             {
@@ -167,14 +203,20 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
                     C.radius();
                     float need = C.rsafe + sqrtf(fmaf(C.rsafe, C.rsafe, dwm));
                     need = need * need * (1.0f + 4e-5f);
+                    const bool base = lo < kLaneShell * dK; // within the first radius
                     if (need <= lo)
                         search = false; // every point within reach was clipped
-                    else if (shell == 2 || (shell == 1 && need > kLaneFar * dK))
+                    else if (shell == 3 || (!base && need > kLaneFar * dK))
                     {
                         C.give_up();
                         search = false;
                     }
-                    hi = shell == 0 ? fminf(need, kLaneShell * dK) : need;
+                    hi = base ? fminf(need, kLaneShell * dK) : need;
+                    if (shell == 0)
+                    {
+                        const float r = hint + sqrtf(fmaf(hint, hint, dwm));
+                        hi = fmaxf(fminf(hi, r * r * (1.0f + 4e-5f)), lo);
+                    }
                 }
                 if (!__any_sync(kFull, search))
                     break;
@@ -210,26 +252,25 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
                         const float4 a0 = pa[0], a1 = pa[1], a2 = pa[2], a3 = pa[3];
                         const float4 b0 = pb[0], b1 = pb[1], b2 = pb[2], b3 = pb[3];
                         sp -= 1 + two;
-                        const bool h0 = __any_sync(kFull, lane_box_dist(C.s, a0.x, a0.y, a0.z, a0.w, a1.x, a1.y) <= rr);
-                        const bool h1 = __any_sync(kFull, lane_box_dist(C.s, a1.z, a1.w, a2.x, a2.y, a2.z, a2.w) <= rr);
-                        const bool h2 =
-                            two && __any_sync(kFull, lane_box_dist(C.s, b0.x, b0.y, b0.z, b0.w, b1.x, b1.y) <= rr);
-                        const bool h3 =
-                            two && __any_sync(kFull, lane_box_dist(C.s, b1.z, b1.w, b2.x, b2.y, b2.z, b2.w) <= rr);
-                        C.n_nodes += rr >= 0.0f ? 2u + 2u * two : 0u;
+                        // (the two children of each; a lane counts those within its own reach)
+                        const bool mine[4] = {lane_box_dist(C.s, a0.x, a0.y, a0.z, a0.w, a1.x, a1.y) <= rr,
+                                              lane_box_dist(C.s, a1.z, a1.w, a2.x, a2.y, a2.z, a2.w) <= rr,
+                                              two && lane_box_dist(C.s, b0.x, b0.y, b0.z, b0.w, b1.x, b1.y) <= rr,
+                                              two && lane_box_dist(C.s, b1.z, b1.w, b2.x, b2.y, b2.z, b2.w) <= rr};
                         if (sp + 4 > kLaneStack)
                         {
                             over = true;
                             sp = 0;
                             break;
                         }
-                        const bool h[4] = {h0, h1, h2, h3};
                         const float f4[4] = {a3.x, a3.y, b3.x, b3.y};
 #pragma unroll
                         for (int c = 0; c < 4; ++c)
-                            if (h[c])
+                            if (__any_sync(kFull, mine[c]))
                             {
                                 const int f = __float_as_int(f4[c]);
+                                C.n_nodes += mine[c] ? 1u : 0u;
+                                C.n_leaves += mine[c] && f < 0 ? 1u : 0u;
                                 if (lane == 0)
                                     (f < 0 ? m.lv[nl] : m.stk[sp]) = f;
                                 nl += f < 0 ? 1 : 0;
@@ -239,7 +280,6 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
                     }
                     if (over)
                         break;
-                    C.n_leaves += rr >= 0.0f ? nl : 0;
                     if (lane == 0)
                         m.lv[nl] = 0; // the last pair may have one leaf
                     __syncwarp();
@@ -305,7 +345,7 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
 #pragma unroll
                         for (int u = 0; u < 4; ++u)
                             if (j[u] >= 0 && ((may >> u) & 1u) &&
-                                !(shell == 0 && j[u] <= jK && lane_sq_dist(C.s, A.pts[j[u]]) == dK)) // (clipped before)
+                                !(!GUESS && shell == 0 && j[u] <= jK && lane_sq_dist(C.s, A.pts[j[u]]) == dK)) // (clipped before)
                             {
                                 if (nk < kLaneCut)
                                     cand[nk] = j[u];
@@ -348,6 +388,8 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
                     }
                     if (q.x == C.s.x && q.y == C.s.y && q.z == C.s.z)
                         continue; // coincident points do not clip each other
+                    if (GUESS && C.has_plane(j))
+                        continue; // clipped before
                     cq = make_cand(C.s, q, j);
                     cut = C.classify(cq, j, r0, r1);
                     if (!C.alive)
@@ -367,6 +409,15 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
             }
         }
         __syncwarp();
+        if (A.hint != nullptr && C.alive && hint < INFINITY)
+        {
+            C.radius();
+            C.n_hit += C.rsafe <= hint ? 1u : 0u;
+            C.n_miss += C.rsafe <= hint ? 0u : 1u;
+        }
+        if (EXPORT && act)
+            C.export_cell();
+        __syncwarp();
         if (act)
             C.output(list, &A.counters[8]);
         __syncwarp();
@@ -380,8 +431,11 @@ void lane_launch(const CellArgs &A, int *list, int num_sms, cudaStream_t st)
 {
     const int64_t need = (A.end - A.begin + 31) / 32;
     const int64_t grid = std::min<int64_t>((int64_t)num_sms * kLaneBlocks, need);
+    const bool exports = A.geometry_out || A.vertices_out || A.vertex_planes_out || A.vertex_count_out;
+    void (*kern)(CellArgs, int *) = A.guesses ? (exports ? k_cells_lane<true, true> : k_cells_lane<true, false>)
+                                              : (exports ? k_cells_lane<false, true> : k_cells_lane<false, false>);
     ++g_launches;
-    k_cells_lane<<<(unsigned)std::max<int64_t>(grid, 1), 32, 0, st>>>(A, list);
+    kern<<<(unsigned)std::max<int64_t>(grid, 1), 32, 0, st>>>(A, list);
 }
 
 } // namespace pg

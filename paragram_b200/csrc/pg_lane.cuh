@@ -99,7 +99,8 @@ struct LaneCell
     unsigned live = 0;       // plane slots that a vertex uses
     float rsafe = INFINITY;  // no vertex lies farther from the seed (after radius())
     // statistics
-    unsigned n_tests = 0, n_nodes = 0, n_leaves = 0, n_clips = 0, n_cands = 0, n_fp64 = 0, n_exp = 0, n_v64 = 0;
+    unsigned n_tests = 0, n_nodes = 0, n_leaves = 0, n_clips = 0, n_cands = 0, n_fp64 = 0, n_exp = 0, n_v64 = 0,
+             n_hit = 0, n_miss = 0;
 #ifdef PG_PHASE_CYCLES
     long long cyc[kLaneCycNum] = {};
 #endif
@@ -192,15 +193,15 @@ struct LaneCell
     // No vertex (with its error bound) lies farther from the seed than rsafe.
     __device__ __forceinline__ void radius()
     {
-        float x2m = 0.0f, pm = 0.0f;
+        float r = 0.0f;
 #pragma unroll 4
         for (int v = 0; v < nv; ++v)
         {
             const float4 X = vxl(v);
-            x2m = fmaxf(x2m, X.x * X.x + X.y * X.y + X.z * X.z);
-            pm = fmaxf(pm, X.w);
+            const float x2 = X.x * X.x + X.y * X.y + X.z * X.z;
+            r = fmaxf(r, (x2 > 0.0f ? x2 * rsqrtf(x2) * (1.0f + 4e-6f) : 0.0f) + X.w);
         }
-        rsafe = (sqrtf(x2m) * (1.0f + 1e-6f) + pm) * (1.0f + 1e-6f);
+        rsafe = r * (1.0f + 1e-6f);
     }
 
     // Which of four candidates may remove a vertex (bit clear: it certainly removes none). One pass over the
@@ -416,6 +417,123 @@ struct LaneCell
         }
     }
 
+    // Whether point j is one of the cell's planes.
+    __device__ __forceinline__ bool has_plane(int j)
+    {
+        bool has = false;
+        for (unsigned w = live; w != 0u; w &= w - 1u)
+            has = has || pidl(__ffs(w) - 1) == j;
+        return has;
+    }
+
+    // Geometry and vertex export of a finished cell, as export_cell of pg_cells.cu: the vertices whose error
+    // radius exceeds 32 ulps are first solved in FP64; the volume is the signed sum of the tetrahedra (o, f_a,
+    // v, u) over the directed edges v -> u of every face a, o the mean vertex and f_a the foot of its
+    // perpendicular on the face. Two vertices share an edge when their triples share two planes; the edge t - u
+    // of t = (a, b, c) and u = (a, c, d) runs t -> u in face a and u -> t in face c.
+    __device__ __forceinline__ void export_cell()
+    {
+        if (defer)
+            return; // the larger pass exports it
+        const bool vertices = A.vertex_count_out != nullptr || A.vertices_out != nullptr || A.vertex_planes_out != nullptr;
+        if (empty)
+        {
+            const float nan = __int_as_float(0x7fc00000);
+            if (A.geometry_out != nullptr)
+                A.geometry_out[soid] = make_float4(nan, nan, nan, 0.0f);
+            if (A.vertex_count_out != nullptr)
+                A.vertex_count_out[soid] = 0;
+            return;
+        }
+        float ox = 0.0f, oy = 0.0f, oz = 0.0f;
+#pragma unroll 1
+        for (int v = 0; v < nv; ++v)
+        {
+            float4 X = vxl(v);
+            if (!(X.w <= 32.0f * kEps * (fabsf(X.x) + fabsf(X.y) + fabsf(X.z))))
+            {
+                const unsigned tr = __float_as_uint(X.w) & 0x7FFFu;
+                X = vertex64_plain(pidl(tr & 31u), pidl((tr >> 5) & 31u), pidl(tr >> 10), A.pts, A.oid, box, s, X);
+                vxl(v) = X;
+            }
+            ox += X.x;
+            oy += X.y;
+            oz += X.z;
+            if (vertices && v < A.vertex_cap)
+            {
+                const size_t at = (size_t)soid * A.vertex_cap + v;
+                if (A.vertices_out != nullptr)
+                    A.vertices_out[at] = X;
+                if (A.vertex_planes_out != nullptr)
+                {
+                    const unsigned tr = __float_as_uint(X.w) & 0x7FFFu;
+#pragma unroll
+                    for (int e = 0; e < 3; ++e)
+                    {
+                        const int id = pidl((tr >> (5 * e)) & 31u);
+                        A.vertex_planes_out[at * 3 + e] = id >= 0 ? A.oid[id] : id;
+                    }
+                }
+            }
+        }
+        if (A.vertex_count_out != nullptr)
+            A.vertex_count_out[soid] = nv;
+        if (A.geometry_out == nullptr)
+            return;
+        const float inv = 1.0f / (float)nv;
+        ox *= inv;
+        oy *= inv;
+        oz *= inv;
+        auto foot = [&](unsigned p) -> float3 {
+            const float4 n = lane_plane(pidl(p), s, A.pts, box).p;
+            const float sc =
+                (n.w - (n.x * ox + n.y * oy + n.z * oz)) / (n.x * n.x + n.y * n.y + n.z * n.z);
+            return make_float3(n.x * sc, n.y * sc, n.z * sc);
+        };
+        double S = 0.0, cx = 0.0, cy = 0.0, cz = 0.0;
+#pragma unroll 1
+        for (int t = 0; t < nv; ++t)
+        {
+            const unsigned tr = tri_of(t), bt = tri_bits(tr);
+            int e0 = -1, e1 = -1, e2 = -1; // the later vertices that share an edge with t
+            for (int u = t + 1; u < nv; ++u)
+                if (__popc(bt & tri_bits(tri_of(u))) == 2)
+                {
+                    e2 = e1;
+                    e1 = e0;
+                    e0 = u;
+                }
+            const float4 T = vxl(t);
+            const float vx = T.x - ox, vy = T.y - oy, vz = T.z - oz;
+            while (e0 >= 0)
+            {
+                const unsigned shared = bt & tri_bits(tri_of(e0));
+                const unsigned p0 = tr & 31u, p1 = (tr >> 5) & 31u, p2 = tr >> 10;
+                unsigned a = p1, c = p0; // b = p2
+                if (!((shared >> p0) & 1u))
+                    a = p2, c = p1;
+                else if (!((shared >> p1) & 1u))
+                    a = p0, c = p2;
+                const float4 U = vxl(e0);
+                const float ux = U.x - ox, uy = U.y - oy, uz = U.z - oz;
+                const float rx = vy * uz - vz * uy, ry = vz * ux - vx * uz, rz = vx * uy - vy * ux;
+                const float3 fa = foot(a), fc = foot(c);
+                const float da = fa.x * rx + fa.y * ry + fa.z * rz, dc = -(fc.x * rx + fc.y * ry + fc.z * rz);
+                S += (double)da + (double)dc;
+                cx += (double)da * (fa.x + vx + ux) + (double)dc * (fc.x + vx + ux);
+                cy += (double)da * (fa.y + vy + uy) + (double)dc * (fc.y + vy + uy);
+                cz += (double)da * (fa.z + vz + uz) + (double)dc * (fc.z + vz + uz);
+                e0 = e1;
+                e1 = e2;
+                e2 = -1;
+            }
+        }
+        const double q = 0.25 / S;
+        A.geometry_out[soid] =
+            make_float4((float)((double)s.x + (double)ox + cx * q), (float)((double)s.y + (double)oy + cy * q),
+                        (float)((double)s.z + (double)oz + cz * q), (float)(fabs(S) / 6.0));
+    }
+
     // Row, degree and status of a finished cell, or its entry in `list` (counted in *list_n).
     __device__ __forceinline__ void output(int *list, int *list_n)
     {
@@ -471,6 +589,8 @@ struct LaneCell
         flush_one(n_fp64, kStatFp64);
         flush_one(n_exp, kStatExpansion);
         flush_one(n_v64, kStatVertex64);
+        flush_one(n_hit, kStatHintHit);
+        flush_one(n_miss, kStatHintMiss);
 #ifdef PG_PHASE_CYCLES
         // (every lane of a warp is in the same phase: each of its cells sees these cycles)
         long long all = 0;

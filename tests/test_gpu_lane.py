@@ -85,3 +85,66 @@ def test_lane_pass_equals_warp_pass_and_chunks(dev):
         got, st = _gpu(p, w, dev, num_chunks=chunks)
         assert all(np.array_equal(x, y) for x, y in zip(got, ref)), chunks
         assert st["clips"] > 10 * len(p)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "heavy", "surface"])
+def test_lane_pass_exports(dev, kind):
+    """Volumes, centroids and vertices of the lane pass against the warp-per-cell pass: the same vertices
+    (each within both passes' bounds) and integrals of them. Both integrate FP32 vertices within 2^-19 of
+    their length; a volume then differs by at most about 3 * 2^-18 times (length / size of the cell)."""
+    p, w = _cloud(kind, 40_000)
+    g0, a = _gpu(p, w, dev, geometry=True, vertices=64, blocks_per_sm=2)
+    g1, b = _gpu(p, w, dev, geometry=True, vertices=64)
+    assert all(np.array_equal(x, y) for x, y in zip(g0, g1))
+    assert torch.equal(a["vertex_count"], b["vertex_count"])
+    va, vb = a["volumes"].double(), b["volumes"].double()
+    full = va > 0
+    assert torch.equal(full, vb > 0)
+    rel = ((va - vb).abs() / va)[full]
+    assert float(rel.median()) < 1e-5 and float((va - vb).norm() / va.norm()) < 2e-5
+    ca, cb = a["centroids"].double()[full], b["centroids"].double()[full]
+    assert float((ca - cb).norm() / ca.norm()) < 2e-5
+    assert torch.equal(torch.isnan(a["centroids"]), torch.isnan(b["centroids"]))
+    # vertex by vertex: matched by their three planes
+    k = min(64, int(a["vertex_count"].max()))
+    pa, pb = a["vertex_planes"][:, :k].sort(2).values, b["vertex_planes"][:, :k].sort(2).values
+    n = len(p)
+    used = (torch.arange(k, device=dev)[None] < a["vertex_count"][:, None]) & (a["vertex_count"][:, None] <= 64)
+    key = lambda q: ((q[..., 0] + 8) * (n + 16) + q[..., 1] + 8) * (n + 16) + q[..., 2] + 8  # noqa: E731
+    big = torch.iinfo(torch.int64).max
+    ka, ia = torch.where(used, key(pa.long()), big).sort(1)
+    kb, ib = torch.where(used, key(pb.long()), big).sort(1)
+    assert torch.equal(ka, kb)
+    xa = torch.gather(a["vertices"][:, :k], 1, ia[..., None].expand(-1, -1, 3)).double()
+    xb = torch.gather(b["vertices"][:, :k], 1, ib[..., None].expand(-1, -1, 3)).double()
+    ba, bb = torch.gather(a["vertex_bound"][:, :k], 1, ia), torch.gather(b["vertex_bound"][:, :k], 1, ib)
+    on = ka < big
+    assert bool(((xa - xb).norm(dim=2)[on] <= (ba + bb)[on].double() * (1 + 1e-6)).all())
+
+
+def test_lane_pass_guesses_and_radius(dev):
+    """Initial guesses (true neighbours, with repeats, the point itself and ids out of range; too many; none)
+    and search radii (exact, far too small, none) leave the diagram as it is."""
+    p, w = _cloud("power", 40_000)
+    n = len(p)
+    (adj, off, st), cold = _gpu(p, w, dev, diagnostics=True)
+    rng = np.random.default_rng(3)
+    rows = [adj[off[u]:off[u + 1]] for u in range(n)]
+    for u in range(0, n, 7):
+        rows[u] = np.concatenate([rows[u][::2], rows[u][:3], [u, -5, n + 9]]).astype(np.int32)
+    for u in range(3, n, 50):
+        rows[u] = rng.integers(0, n, 60).astype(np.int32)
+    for u in range(5, n, 50):
+        rows[u] = rows[u][:0]
+    go = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+    g = torch.from_numpy(np.concatenate(rows).astype(np.int32)).to(dev)
+    guesses = dict(initial_guesses=g, initial_guesses_offsets=torch.from_numpy(go).to(dev))
+    radius = cold["radius"]
+    for kw in (guesses, dict(radius_hint=radius * 1.0001), dict(radius_hint=radius * 0.3),
+               dict(radius_hint=radius * 1.0001, **guesses)):
+        got, stats = _gpu(p, w, dev, **kw)
+        assert all(np.array_equal(x, y) for x, y in zip(got, (adj, off, st))), list(kw)
+        if "radius_hint" in kw:
+            hits, misses = stats["hint_hits"], stats["hint_misses"]
+            exact = kw["radius_hint"][0] > radius[0]
+            assert hits + misses > 0.8 * n and (misses == 0 if exact else misses > 0.9 * (hits + misses))
