@@ -4,16 +4,15 @@
 // the point itself (pwr_bvh.cu:159-215); it warm-starts every cell with them
 // (voronoi_ultra.cu:205-227). Here the query runs on the LBVH of pg_build
 // (pg_lbvh.cu): one thread per sorted slot (neighbouring threads query
-// neighbouring points, so their traversals share nodes in L1/L2), a
-// depth-first descent into the nearer child first with a fixed stack, the k
-// best kept sorted by (squared distance, original index). Distances are the
-// unweighted Euclidean ones in FP32 (like the reference's, also for power
-// diagrams), each product and sum rounded separately so that a CPU restatement
+// neighbouring points, so their traversals share nodes in L1/L2), upwards from
+// the point's own leaf, the k best kept sorted by (squared distance, original
+// index). Distances are the unweighted Euclidean ones in FP32 (like the
+// reference's, also for power diagrams), each product and sum rounded separately so that a CPU restatement
 // in float32 reproduces them and their ties exactly. A point's copies at the
 // same position are neighbours like any other point; only its own index is
-// excluded. The cell pass does not use the result (its traversal starts at the
-// point's own leaf); pg_knn exports it, and the Python layer can pass it to a
-// build as initial guesses, which is the reference's warm start.
+// excluded. The cell-per-lane pass clips its cells by the result first; pg_knn
+// exports it, and the Python layer can pass it to a build as initial guesses,
+// which is the reference's warm start.
 #include <algorithm>
 #include <string>
 
@@ -49,96 +48,26 @@ __device__ __forceinline__ float box_sq_dist(float4 q, float lx, float ly, float
     return (dx * dx + dy * dy + dz * dz) * (1.0f - 1e-5f);
 }
 
-__global__ void __launch_bounds__(128) k_knn(int64_t n, int k, const float4 *__restrict__ pts,
+// The K nearest other points of sorted slots [begin, end), nearest first. Starts at the point's own leaf and
+// climbs to the cloud's root, searching each sibling subtree within the K-th distance so far. The list lives in
+// registers as (distance bits, id) keys, unrolled: with a dynamically indexed array, which lives in local
+// memory, and a descent from the root, 8 neighbours of 1M clustered points took 1.81 ms; 1.28 here (the key
+// ROWS (the cell pass): ids are sorted slots, written to the cells' rows (-1 beyond the cloud's points, -2 when
+// the descent outgrew its stack). Else (pg_knn): ids are original indices, the first k of the list written.
+template <int K, bool ROWS>
+__global__ void __launch_bounds__(128) k_knn(int64_t begin, int64_t end, const float4 *__restrict__ pts,
                                              const int *__restrict__ oid, const float4 *__restrict__ rec,
+                                             const int *__restrict__ rparent, const int *__restrict__ pleaf,
                                              const int *__restrict__ cloud_off, int num_clouds,
-                                             const int *__restrict__ cloud_root, int *__restrict__ out, int *err)
-{
-    int64_t ii = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (ii >= n)
-        return;
-    const int i = (int)ii;
-    const float4 q = pts[i];
-    const int root = cloud_root[cloud_of(cloud_off, num_clouds, i)];
-    float bd[kKnnMax];
-    int bi[kKnnMax];
-    int cnt = 0;
-    int stk[kKnnStack];
-    float skey[kKnnStack];
-    int sp = 0;
-    stk[sp] = root;
-    skey[sp++] = 0.0f;
-    while (sp > 0)
-    {
-        --sp;
-        const int ref = stk[sp];
-        const float key = skey[sp];
-        const float worst = cnt < k ? INFINITY : bd[k - 1];
-        if (key > worst)
-            continue;
-        if (ref < 0)
-        {
-            for (int j = leaf_first(ref), e = j + leaf_count(ref); j < e; ++j)
-            {
-                if (j == i)
-                    continue;
-                const float d = sq_dist(q, pts[j]);
-                const int id = oid[j];
-                if (cnt == k && (d > bd[k - 1] || (d == bd[k - 1] && id > bi[k - 1])))
-                    continue;
-                // insertion into the sorted list (the last entry drops out when it is full)
-                int at = cnt < k ? cnt++ : k - 1;
-                while (at > 0 && (bd[at - 1] > d || (bd[at - 1] == d && bi[at - 1] > id)))
-                {
-                    bd[at] = bd[at - 1];
-                    bi[at] = bi[at - 1];
-                    --at;
-                }
-                bd[at] = d;
-                bi[at] = id;
-            }
-            continue;
-        }
-        const float4 *r = rec + 4 * (size_t)ref;
-        const float4 r0 = r[0], r1 = r[1], r2 = r[2], r3 = r[3];
-        const float k0 = box_sq_dist(q, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y);
-        const float k1 = box_sq_dist(q, r1.z, r1.w, r2.x, r2.y, r2.z, r2.w);
-        const int c0 = __float_as_int(r3.x), c1 = __float_as_int(r3.y);
-        if (sp + 2 > kKnnStack)
-        {
-            atomicExch(err, 3);
-            break;
-        }
-        // the nearer child is popped first
-        const bool near0 = k0 <= k1;
-        stk[sp] = near0 ? c1 : c0;
-        skey[sp++] = near0 ? k1 : k0;
-        stk[sp] = near0 ? c0 : c1;
-        skey[sp++] = near0 ? k0 : k1;
-    }
-    int *o = out + (size_t)oid[i] * k;
-    for (int t = 0; t < k; ++t)
-        o[t] = t < cnt ? bi[t] : -1;
-}
-
-// The K nearest other points of sorted slots [begin, end), nearest first, as sorted slots into the
-// cells' rows (-1 beyond the cloud's points, -2 when the descent outgrew its stack); ties by slot. Starts at the point's own leaf and climbs
-// to the cloud's root, searching each sibling subtree within the K-th distance so far. The list lives
-// in registers as (distance bits, slot) keys (dynamically indexed arrays live in local memory: the plain
-// query's 8 points take 8.3 ms at 5M clustered points, these 16 take 10.1).
-template <int K>
-__global__ void __launch_bounds__(128) k_knn_rows(int64_t begin, int64_t end, const float4 *__restrict__ pts,
-                                                  const int *__restrict__ oid, const float4 *__restrict__ rec,
-                                                  const int *__restrict__ rparent, const int *__restrict__ pleaf,
-                                                  const int *__restrict__ cloud_off, int num_clouds,
-                                                  const int *__restrict__ cloud_root, int *__restrict__ rows)
+                                             const int *__restrict__ cloud_root, int *__restrict__ out, int k,
+                                             int *err)
 {
     const int64_t ii = begin + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool alive = ii < end;
     const int i = (int)(alive ? ii : end - 1);
     const float4 q = pts[i];
     const int root = cloud_root[cloud_of(cloud_off, num_clouds, i)];
-    alive = alive && root >= 0; // (a cloud of one leaf has no records; its cells do not use this)
+    auto dist = [&](float4 p) -> float { return ROWS ? lane_sq_dist(q, p) : sq_dist(q, p); };
     unsigned long long best[K];
 #pragma unroll
     for (int t = 0; t < K; ++t)
@@ -146,11 +75,12 @@ __global__ void __launch_bounds__(128) k_knn_rows(int64_t begin, int64_t end, co
     float worst = INFINITY;
     int stk[kKnnStack];
     int sp = 0;
-    int e = alive ? pleaf[i] : -1; // entry (parent << 1 | side) of the path node whose subtree is done
-    int leaf = 0;
+    int e = -1; // entry (parent << 1 | side) of the path node whose subtree is done
+    int leaf = alive ? root : 0; // (a cloud of one leaf has no records)
     bool full = false;
-    if (alive)
+    if (alive && root >= 0)
     {
+        e = pleaf[i];
         const float4 r3 = rec[4 * (size_t)(e >> 1) + 3];
         leaf = __float_as_int((e & 1) ? r3.y : r3.x);
     }
@@ -208,13 +138,13 @@ __global__ void __launch_bounds__(128) k_knn_rows(int64_t begin, int64_t end, co
             leaf = 0;
             unsigned todo = 0u;
             for (int p = 0; p < count; ++p)
-                if (first + p != i && lane_sq_dist(q, pts[first + p]) <= worst)
+                if (first + p != i && dist(pts[first + p]) <= worst)
                     todo |= 1u << p;
             for (; todo != 0u; todo &= todo - 1u)
             {
                 const int j = first + __ffs(todo) - 1;
                 const unsigned long long key =
-                    ((unsigned long long)__float_as_uint(lane_sq_dist(q, pts[j])) << 32) | (unsigned)j;
+                    ((unsigned long long)__float_as_uint(dist(pts[j])) << 32) | (unsigned)(ROWS ? j : oid[j]);
                 bool below = key < best[K - 1];
 #pragma unroll
                 for (int t = K - 1; t > 0; --t)
@@ -229,13 +159,15 @@ __global__ void __launch_bounds__(128) k_knn_rows(int64_t begin, int64_t end, co
         }
         __syncwarp();
     }
-    if (ii < end)
-    {
-        int *o = rows + (size_t)oid[i] * kRowWidth;
+    if (ii >= end)
+        return;
+    if (!ROWS && full)
+        atomicExch(err, 3);
+    int *o = out + (size_t)oid[i] * (ROWS ? kRowWidth : k);
 #pragma unroll
-        for (int t = 0; t < K; ++t)
-            o[t] = full ? -2 : (best[t] == ~0ull ? -1 : (int)(unsigned)best[t]);
-    }
+    for (int t = 0; t < K; ++t)
+        if (ROWS || t < k)
+            o[t] = ROWS && full ? -2 : (best[t] == ~0ull ? -1 : (int)(unsigned)best[t]);
 }
 
 void knn_rows_launch(const Workspace &ws, int num_clouds, int64_t begin, int64_t end, cudaStream_t st)
@@ -243,9 +175,9 @@ void knn_rows_launch(const Workspace &ws, int num_clouds, int64_t begin, int64_t
     if (end <= begin)
         return;
     ++g_launches;
-    k_knn_rows<kLaneWarm><<<(unsigned)((end - begin + 127) / 128), 128, 0, st>>>(
+    k_knn<kLaneWarm, true><<<(unsigned)((end - begin + 127) / 128), 128, 0, st>>>(
         begin, end, ws.pts, ws.oid, ws.records, ws.rparent, ws.pleaf, ws.cloud_off, num_clouds, ws.cloud_root,
-        ws.rows);
+        ws.rows, kLaneWarm, nullptr);
 }
 
 } // namespace pg
@@ -276,9 +208,28 @@ extern "C" int pg_knn(int64_t num_points, const float *points, int32_t k, void *
     k_knn_single_cloud<<<1, 1, 0, st>>>(ws.cloud_off, (int)num_points);
     lbvh_build(ws, num_points, 1, points, nullptr, kDefaultLeaf, st);
     ++g_launches;
-    k_knn<<<(unsigned)((num_points + 127) / 128), 128, 0, st>>>(num_points, k, ws.pts, ws.oid, ws.records,
-                                                                ws.cloud_off, 1, ws.cloud_root, neighbours,
-                                                                &ws.counters[2]);
+    // the smallest list that holds k (its length prunes the search)
+    auto run = [&](auto kern) {
+        kern<<<(unsigned)((num_points + 127) / 128), 128, 0, st>>>(0, num_points, ws.pts, ws.oid, ws.records,
+                                                                   ws.rparent, ws.pleaf, ws.cloud_off, 1,
+                                                                   ws.cloud_root, neighbours, k, &ws.counters[2]);
+    };
+    if (k <= 2)
+        run(k_knn<2, false>);
+    else if (k <= 4)
+        run(k_knn<4, false>);
+    else if (k <= 6)
+        run(k_knn<6, false>);
+    else if (k <= 8)
+        run(k_knn<8, false>);
+    else if (k <= 12)
+        run(k_knn<12, false>);
+    else if (k <= 16)
+        run(k_knn<16, false>);
+    else if (k <= 24)
+        run(k_knn<24, false>);
+    else
+        run(k_knn<32, false>);
     int flag = 0;
     cudaMemcpyAsync(&flag, &ws.counters[2], sizeof(int), cudaMemcpyDeviceToHost, st);
     cudaError_t e = cudaStreamSynchronize(st);

@@ -9,7 +9,7 @@
 // them: 8,100 for 32 cells' steps per cell.
 //
 // What keeps the lanes in step: (1) a cell is first clipped by its kLaneWarm nearest
-// points (k_knn_rows), nearly all of which cut it; (2) the points that can still
+// points (k_knn), nearly all of which cut it; (2) the points that can still
 // reach it come from one search of the BVH for the warp's 32 cells, whose nodes and
 // leaves every lane tests at the same time; (3) the points in reach are tested four
 // at a time against the vertices, and only those that may cut (about 8 of 50) are

@@ -69,7 +69,7 @@ __device__ __forceinline__ LPlane lane_plane(int pid, float4 s, const float4 *__
     return r;
 }
 
-// Squared distance of two points; k_knn_rows and the cell pass compute it alike, so that they agree exactly.
+// Squared distance of two points; k_knn and the cell pass compute it alike, so that they agree exactly.
 __device__ __forceinline__ float lane_sq_dist(float4 a, float4 b)
 {
     const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;

@@ -79,3 +79,19 @@ def test_knn_warm_start_same_diagram(dev, oracle):
     a = pg.voronoi_diagram(tc)
     b = pg.voronoi_diagram(tc, knn=8, knn_warm_start=True)
     assert torch.equal(a.adjacency, b.adjacency) and torch.equal(a.status, b.status)
+
+
+@pytest.mark.parametrize("k", [2, 3, 4, 5, 6, 7, 9, 12, 13, 16, 17, 24, 25])
+def test_knn_list_lengths(dev, k):
+    """The query's list lengths: every k around the lengths that the kernel is built for."""
+    import paragram_b200 as pg
+
+    rng = np.random.default_rng(k)
+    pts = rng.random((600, 3), dtype=np.float32)
+    pts[100:140] = pts[100]  # ties, decided by index
+    got = pg.knn(torch.from_numpy(pts).to(dev), k).cpu().numpy()
+    d = ((pts[:, None, 0] - pts[None, :, 0]) ** 2 + (pts[:, None, 1] - pts[None, :, 1]) ** 2) + \
+        (pts[:, None, 2] - pts[None, :, 2]) ** 2
+    d[np.arange(600), np.arange(600)] = np.inf
+    exp = np.lexsort((np.broadcast_to(np.arange(600), d.shape), d), axis=1)[:, :k]
+    assert np.array_equal(got, exp)
