@@ -51,7 +51,8 @@ __device__ __forceinline__ float box_sq_dist(float4 q, float lx, float ly, float
 // The K nearest other points of sorted slots [begin, end), nearest first. Starts at the point's own leaf and
 // climbs to the cloud's root, searching each sibling subtree within the K-th distance so far. The list lives in
 // registers as (distance bits, id) keys, unrolled: with a dynamically indexed array, which lives in local
-// memory, and a descent from the root, 8 neighbours of 1M clustered points took 1.81 ms; 1.28 here (the key
+// memory, and a descent from the root, 8 neighbours of 1M clustered points took 1.81 ms; 1.28 here,
+// bound by the ALU (64-bit compares and selects of the insertions).
 // ROWS (the cell pass): ids are sorted slots, written to the cells' rows (-1 beyond the cloud's points, -2 when
 // the descent outgrew its stack). Else (pg_knn): ids are original indices, the first k of the list written.
 template <int K, bool ROWS>
