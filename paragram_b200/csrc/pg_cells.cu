@@ -83,6 +83,7 @@ template <int CAP, int STACK> struct CellMem
     float cap;  // search radius of the current pass (learned / given; +inf without one)
     float done; // search radius of the finished first pass (-inf during the first pass)
     unsigned et[CAP * CAP / 32];       // edge table of the clip in progress (all zero between clips)
+    typename std::conditional<(CAP <= 256), unsigned char, unsigned short>::type rl[CAP]; // its removed slots, by rank
 };
 
 // Clear a warp's edge table (once, before its first clip).
@@ -299,20 +300,27 @@ enum ClipResult : int
     kClipDefer = 3,
 };
 
+// Clip by one candidate. The removed slots are listed by rank, so that what follows the vertex tests is a
+// handful of steps for any number of vertex words: lane r takes the r-th removed vertex (its edges marked,
+// tested, listed by ballots), then the r-th boundary edge (in the r-th removed slot, then in free ones).
+// Listing edges and searching slots word by word instead cost the larger tiers, whose time is the chain of
+// their slowest cells, 39.7 ms in the 256-slot tier of 24 surface clouds (25.7 so) and 8.0 in the 128-slot
+// tier (7.0); the 64-slot pass takes 21.8 against 21.2 ms there.
 template <int CAP, int STACK>
-__device__ __forceinline__ int clip(CellMem<CAP, STACK> &m, WarpState<CAP> &ws, const Cand &q, const CellArgs &A, int lane)
+__device__ __forceinline__ int clip(CellMem<CAP, STACK> &m, WarpState<CAP> &ws, const Cand &q, const CellArgs &A,
+                                           int lane)
 {
     constexpr int W = CAP / 32;
+    const unsigned lt = (1u << lane) - 1u;
     unsigned rem[W];
-    unsigned tri[W];
+    int nr = 0, nvalid = 0; // removed, valid vertices
 #pragma unroll(CAP > 256 ? 1 : CAP / 32)
     for (int k = 0; k < W; ++k)
     {
         int r = 0;
-        tri[k] = 0;
+        const int slot = k * 32 + lane;
         if ((ws.valid[k] >> lane) & 1u)
         {
-            int slot = k * 32 + lane;
             float4 X = m.vx[slot];
             r = side_fp32(X, q);
             if (r < 0 && A.fp32_only)
@@ -332,22 +340,17 @@ __device__ __forceinline__ int clip(CellMem<CAP, STACK> &m, WarpState<CAP> &ws, 
                     r = 0;
                 }
             }
-            if (r)
-                tri[k] = m.vt[slot];
         }
         rem[k] = __ballot_sync(kFull, r == 1);
+        if (r == 1)
+            m.rl[nr + __popc(rem[k] & lt)] = slot;
+        nr += __popc(rem[k]);
+        nvalid += __popc(ws.valid[k]);
     }
-    PG_COUNT(m, lane, kStatTests, count_bits(ws.valid));
-    bool any = false, all = true;
-#pragma unroll(CAP > 256 ? 1 : CAP / 32)
-    for (int k = 0; k < W; ++k)
-    {
-        any = any || rem[k] != 0u;
-        all = all && rem[k] == ws.valid[k];
-    }
-    if (!any)
+    PG_COUNT(m, lane, kStatTests, nvalid);
+    if (nr == 0)
         return kClipNone;
-    if (all)
+    if (nr == nvalid)
     {
         ws.flags |= kFlagEmpty;
 #pragma unroll(CAP > 256 ? 1 : CAP / 32)
@@ -360,164 +363,131 @@ __device__ __forceinline__ int clip(CellMem<CAP, STACK> &m, WarpState<CAP> &ws, 
         gc_planes(m, ws, lane);
         if (ws.np >= CAP)
             return kClipDefer;
-        // plane slots were renumbered: reload the removed triangles
-#pragma unroll(CAP > 256 ? 1 : CAP / 32)
-        for (int k = 0; k < W; ++k)
-            if ((rem[k] >> lane) & 1u)
-                tri[k] = m.vt[k * 32 + lane];
     }
-    int P = ws.np++;
+    const int P = ws.np++;
     if (lane == 0)
     {
         m.pl[P] = make_float4(q.nx, q.ny, q.nz, q.h);
         m.pe[P] = q.eh;
         m.pid[P] = q.id;
     }
-    // boundary edges of the removed region: the directed edge x->y of a removed
-    // triangle is a boundary edge iff y->x is not an edge of another removed
-    // triangle. The removed triangles mark their edges in the warp's edge table
-    // (bit x * CAP + y), each lane tests the reverses of its own edges, then the
-    // marks are cleared (the table is all zero between clips).
-    using Bits = typename std::conditional<(3 * W > 32), unsigned long long, unsigned>::type;
-    Bits bf = 0; // bit k*3+e: edge e of my removed vertex in word k is a boundary edge
-#pragma unroll(CAP > 256 ? 1 : CAP / 32)
-    for (int k = 0; k < W; ++k)
-        if ((rem[k] >> lane) & 1u)
+    __syncwarp();
+    for (int r0 = 0; r0 < nr; r0 += 32)
+        if (r0 + lane < nr)
         {
-            unsigned t = tri[k];
+            const unsigned t = m.vt[m.rl[r0 + lane]];
 #pragma unroll
             for (int e = 0; e < 3; ++e)
             {
-                unsigned bit = tri_get(t, e) * CAP + tri_get(t, (e + 1) % 3);
+                const unsigned bit = tri_get(t, e) * CAP + tri_get(t, (e + 1) % 3);
                 atomicOr(&m.et[bit >> 5], 1u << (bit & 31u));
             }
         }
     __syncwarp();
-#pragma unroll(CAP > 256 ? 1 : CAP / 32)
-    for (int k = 0; k < W; ++k)
-        if ((rem[k] >> lane) & 1u)
-        {
-            unsigned t = tri[k];
+    int nb = 0;
+    for (int r0 = 0; r0 < nr; r0 += 32)
+    {
+        const bool mine = r0 + lane < nr;
+        const unsigned t = mine ? m.vt[m.rl[r0 + lane]] : 0u;
 #pragma unroll
-            for (int e = 0; e < 3; ++e)
-            {
-                unsigned rbit = tri_get(t, (e + 1) % 3) * CAP + tri_get(t, e);
-                if (!((m.et[rbit >> 5] >> (rbit & 31u)) & 1u))
-                    bf |= (Bits)1u << (3 * k + e);
-            }
-        }
-    __syncwarp();
-#pragma unroll(CAP > 256 ? 1 : CAP / 32)
-    for (int k = 0; k < W; ++k)
-        if ((rem[k] >> lane) & 1u)
+        for (int e = 0; e < 3; ++e)
         {
-            unsigned t = tri[k];
+            const unsigned x = tri_get(t, e), y = tri_get(t, (e + 1) % 3);
+            const unsigned rbit = y * CAP + x;
+            const bool edge = mine && !((m.et[rbit >> 5] >> (rbit & 31u)) & 1u);
+            const unsigned b = __ballot_sync(kFull, edge);
+            const int at = nb + __popc(b & lt);
+            if (edge && at < CAP)
+                m.eb[at] = x | (y << 16);
+            nb += __popc(b);
+        }
+    }
+    __syncwarp();
+    for (int r0 = 0; r0 < nr; r0 += 32)
+        if (r0 + lane < nr)
+        {
+            const unsigned t = m.vt[m.rl[r0 + lane]];
 #pragma unroll
             for (int e = 0; e < 3; ++e)
                 m.et[(tri_get(t, e) * CAP + tri_get(t, (e + 1) % 3)) >> 5] = 0u;
         }
-    // list the boundary edges in the warp's edge buffer, lane by lane (exclusive scan of the counts)
-    int mine = 0;
-    if constexpr (3 * W > 32)
-        mine = __popcll(bf);
-    else
-        mine = __popc((unsigned)bf);
-    int incl = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1)
-    {
-        int v = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o)
-            incl += v;
-    }
-    const int nb = __shfl_sync(kFull, incl, 31);
-    {
-        int at = incl - mine;
-#pragma unroll(W > 8 ? 1 : 3 * W)
-        for (int f = 0; f < 3 * W; ++f)
-            if ((bf >> f) & 1u)
-            {
-                unsigned my = tri[f / 3];
-                m.eb[at++] = tri_get(my, f % 3) | (tri_get(my, (f % 3 + 1) % 3) << 16);
-            }
-    }
-    int nv_new = count_bits(ws.valid) - count_bits(rem) + nb;
-    if (nv_new > CAP)
+    if (nvalid - nr + nb > CAP)
         return kClipDefer;
-    unsigned fr[W];
-#pragma unroll(CAP > 256 ? 1 : CAP / 32)
-    for (int k = 0; k < W; ++k)
-        fr[k] = ~ws.valid[k] | rem[k];
-    __syncwarp(); // edge list, plane P and all reads of removed triangles are done
-    float4 pP = m.pl[P];
-    float eP = m.pe[P];
-    unsigned nbits[W];
-#pragma unroll(CAP > 256 ? 1 : CAP / 32)
-    for (int k = 0; k < W; ++k)
-        nbits[k] = 0;
-    bool ill = false; // a vertex built by this lane needs the FP64 rebuild
-    // lane r builds the vertex (P, x, y) of the r-th boundary edge in the r-th free slot
+    __syncwarp(); // all reads of removed triangles are done
+    const float4 pP = m.pl[P];
+    const float eP = m.pe[P];
     for (int r0 = 0; r0 < nb; r0 += 32)
     {
-        int r = r0 + lane;
+        const int r = r0 + lane;
+        bool ill = false;
+        int slot = 0;
+        unsigned x = 0, y = 0;
+        float4 X = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float vr = 0.0f;
         if (r < nb)
         {
-            unsigned xy = m.eb[r];
-            unsigned x = xy & 0xFFFFu, y = xy >> 16;
-            int rr = r, slot = -1;
-#pragma unroll(CAP > 256 ? 1 : CAP / 32)
-            for (int k = 0; k < W; ++k)
+            const unsigned xy = m.eb[r];
+            x = xy & 0xFFFFu;
+            y = xy >> 16;
+            if (r < nr)
+                slot = m.rl[r];
+            else
             {
-                int c = __popc(fr[k]);
-                if (slot < 0 && rr < c)
-                    slot = k * 32 + (int)__fns(fr[k], 0, rr + 1);
-                else if (slot < 0)
-                    rr -= c;
-            }
-            if (slot >= 0 && slot < CAP)
-            {
-                float vr;
-                float4 X = make_vertex(pP, eP, m.pl[x], m.pe[x], m.pl[y], m.pe[y], vr);
-                ill = ill || !(X.w <= kVertex64Rel * (fabsf(X.x) + fabsf(X.y) + fabsf(X.z)));
-                m.vx[slot] = X;
-                m.vr[slot] = vr;
-                m.vt[slot] = tri_pack((unsigned)P, x, y);
+                int u = r - nr; // the u-th free slot
+                slot = -1;
 #pragma unroll(CAP > 256 ? 1 : CAP / 32)
                 for (int k = 0; k < W; ++k)
-                    if ((slot >> 5) == k)
-                        nbits[k] |= 1u << (slot & 31);
-            }
-            else
-                ws.flags |= kFlagError; // unreachable: capacity was checked above
-        }
-    }
-    // ill-conditioned in FP32: rebuild in FP64 so that the empty sphere stays tight
-    if (__any_sync(kFull, ill))
-    {
-#pragma unroll(CAP > 256 ? 1 : CAP / 32)
-        for (int k = 0; k < W; ++k)
-        {
-            unsigned mm = nbits[k];
-            while (mm)
-            {
-                int slot = k * 32 + __ffs(mm) - 1;
-                mm &= mm - 1;
-                float4 X = m.vx[slot];
-                if (!(X.w <= kVertex64Rel * (fabsf(X.x) + fabsf(X.y) + fabsf(X.z))))
                 {
-                    unsigned t = m.vt[slot];
-                    float vr = m.vr[slot];
-                    m.vx[slot] = make_vertex64(m.pid[tri_get(t, 0)], m.pid[tri_get(t, 1)], m.pid[tri_get(t, 2)], A.pts, A.oid,
-                                               ws.box, ws.s, X, vr, vr);
-                    m.vr[slot] = vr;
-                    atomicAdd(&m.cnt[kStatVertex64], 1ull);
+                    unsigned f = ~ws.valid[k];
+                    const int c = __popc(f);
+                    if (slot < 0 && u < c)
+                    {
+                        for (int v = 0; v < u; ++v)
+                            f &= f - 1u;
+                        slot = k * 32 + __ffs(f) - 1;
+                    }
+                    u -= c;
                 }
             }
+            X = make_vertex(pP, eP, m.pl[x], m.pe[x], m.pl[y], m.pe[y], vr);
+            ill = !(X.w <= kVertex64Rel * (fabsf(X.x) + fabsf(X.y) + fabsf(X.z)));
+        }
+        // ill-conditioned in FP32: rebuilt in FP64 so that the empty sphere stays tight
+        if (ill)
+        {
+            X = make_vertex64(m.pid[P], m.pid[x], m.pid[y], A.pts, A.oid, ws.box, ws.s, X, vr, vr);
+            atomicAdd(&m.cnt[kStatVertex64], 1ull);
+        }
+        if (r < nb)
+        {
+            m.vx[slot] = X;
+            m.vr[slot] = vr;
+            m.vt[slot] = tri_pack((unsigned)P, x, y);
         }
     }
+    // slots in use: the first nb - nr free ones as well, or less the last nr - nb removed ones
+    int more = nb - nr, pre = 0;
 #pragma unroll(CAP > 256 ? 1 : CAP / 32)
     for (int k = 0; k < W; ++k)
-        ws.valid[k] = (ws.valid[k] & ~rem[k]) | __reduce_or_sync(kFull, nbits[k]);
+    {
+        if (nb >= nr)
+            while (more > 0 && ws.valid[k] != 0xFFFFFFFFu)
+            {
+                ws.valid[k] |= ws.valid[k] + 1u;
+                --more;
+            }
+        else
+        {
+            const int c = __popc(rem[k]);
+            for (int u = max(nb - pre, 0); u < c; ++u)
+            {
+                const unsigned top = 0x80000000u >> __clz(rem[k]);
+                rem[k] &= ~top;
+                ws.valid[k] &= ~top;
+            }
+            pre += c;
+        }
+    }
     __syncwarp();
     PG_COUNT(m, lane, kStatClips, 1);
     return kClipChanged;
@@ -1373,37 +1343,32 @@ __device__ __forceinline__ void cells_body(CellMem<CAP, STACK> &m, const CellArg
     if (lane < kNumStats)
         m.cnt[lane] = 0;
     clear_edges(m, lane);
-    int64_t count = A.big_pass ? min((int64_t)A.counters[1], A.big_cap) : (A.end - A.begin);
-    int *ctr = A.big_pass ? &A.counters[3] : &A.counters[0];
+    const int64_t count = A.end - A.begin;
     for (;;)
     {
         int t = 0;
         if (lane == 0)
-            t = atomicAdd(ctr, 1);
+            t = atomicAdd(&A.counters[0], 1);
         t = __shfl_sync(kFull, t, 0);
         if (t >= count)
             break;
-        int i = A.big_pass ? A.big_list[t] : (int)(A.begin + t);
+        int i = (int)(A.begin + t);
         // a cell the learned model routed to the 128-slot tier (listed by the prediction)
         if (HINT && A.hint != nullptr && A.hint[i] < 0.0f)
             continue;
         PG_T0(tcell);
         process_cell<CAP, STACK, GUESS, HINT>(m, ws, i, A, lane);
         write_diagnostics(m, ws, A, lane);
-        if (A.big_pass)
-            ws.si = t; // the deferred-row slot
         if (__any_sync(kFull, ws.flags & kFlagError)) // a flag may be set on any lane
         {
             if (lane == 0)
                 atomicExch(&A.counters[2], 1);
             ws.flags &= ~kFlagError;
         }
-        if (A.big_pass && (ws.flags & kFlagDefer) && ws.si < A.big_cap && huge_cell(A, i, lane, ws.si))
-            continue; // outgrew the 256 slots too: rebuilt with 512
-        if (!(ws.flags & kFlagDefer) || A.big_pass)
+        if (!(ws.flags & kFlagDefer))
         {
             PG_T0(to);
-            bool done = write_outputs(m, ws, A, lane, A.big_pass != 0);
+            bool done = write_outputs(m, ws, A, lane, false);
             PG_T1(m, lane, kStatCycOut, to);
             if (done)
             {
@@ -1611,7 +1576,6 @@ static CellArgs make_args(const Workspace &ws, const CellLaunch &cl)
     A.begin = cl.cell_begin;
     A.end = cl.cell_end;
     A.list = nullptr;
-    A.big_pass = 0;
     A.big_cap = 0;
     A.huge_slabs = (char *)ws.huge_slabs;
     A.radius_out = cl.radius_out;

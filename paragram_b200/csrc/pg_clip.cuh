@@ -44,7 +44,6 @@ struct CellArgs
     int *counters;
     unsigned long long *stats;
     int64_t begin, end;
-    int big_pass;
     const int *list; // cells that the cell-per-lane pass left (sorted slots; their number in counters[8])
     int64_t big_cap;
     char *huge_slabs;
