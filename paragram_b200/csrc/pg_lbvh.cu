@@ -44,36 +44,35 @@ __global__ void k_bounds_init(int *b, int num_clouds)
     b[t] = float_to_ordered(k < 3 ? INFINITY : -INFINITY);
 }
 
-// Per-cloud bounds: warps reduce per distinct cloud (normally one) before the atomics.
-__global__ void k_bounds(const float *__restrict__ p, const float *__restrict__ w, int64_t n,
-                         const int *__restrict__ coff, int num_clouds, int *b)
+// Per-cloud bounds. A block takes a contiguous range; every thread keeps the bounds of its points of one cloud
+// (normally all of them) and a warp's are reduced per distinct cloud when one of its threads meets another
+// cloud, and at the end. (A reduction and seven atomics per 32 points: 0.72 ms at 5M points; 0.057 now.)
+__global__ void __launch_bounds__(256) k_bounds(const float *__restrict__ p, const float *__restrict__ w, int64_t n,
+                                                const int *__restrict__ coff, int num_clouds, int *b)
 {
     const unsigned full = 0xFFFFFFFFu;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x)
-    {
-        int64_t i = base + threadIdx.x;
-        bool ok = i < n;
-        int c = ok ? cloud_of(coff, num_clouds, (int)i) : -1;
-        float v[7] = {0, 0, 0, 0, 0, 0, 0};
-        if (ok)
-        {
-            v[0] = v[3] = p[i * 3 + 0];
-            v[1] = v[4] = p[i * 3 + 1];
-            v[2] = v[5] = p[i * 3 + 2];
-            v[6] = w ? w[i] : 0.0f;
-        }
-        unsigned todo = __ballot_sync(full, ok);
+    const int64_t per = ((n + gridDim.x - 1) / gridDim.x + blockDim.x - 1) / blockDim.x * blockDim.x;
+    const int64_t begin = (int64_t)blockIdx.x * per, end = min(n, begin + per);
+    int c = -1; // the cloud of v
+    float v[7];
+    auto reset = [&]() {
+#pragma unroll
+        for (int k = 0; k < 7; ++k)
+            v[k] = k < 3 ? INFINITY : -INFINITY;
+    };
+    auto flush = [&](bool mine_too) {
+        unsigned todo = __ballot_sync(full, mine_too && c >= 0);
         while (todo)
         {
-            int leader = __ffs(todo) - 1;
-            int cl = __shfl_sync(full, c, leader);
-            bool mine = ok && c == cl;
+            const int leader = __ffs(todo) - 1;
+            const int cl = __shfl_sync(full, c, leader);
+            const bool mine = mine_too && c == cl;
             todo &= ~__ballot_sync(full, mine);
 #pragma unroll
             for (int k = 0; k < 7; ++k)
             {
-                int key = float_to_ordered(mine ? v[k] : (k < 3 ? INFINITY : -INFINITY));
-                int r = k < 3 ? __reduce_min_sync(full, key) : __reduce_max_sync(full, key);
+                const int key = float_to_ordered(mine ? v[k] : (k < 3 ? INFINITY : -INFINITY));
+                const int r = k < 3 ? __reduce_min_sync(full, key) : __reduce_max_sync(full, key);
                 if ((int)(threadIdx.x & 31) == leader)
                 {
                     if (k < 3)
@@ -83,7 +82,34 @@ __global__ void k_bounds(const float *__restrict__ p, const float *__restrict__ 
                 }
             }
         }
+    };
+    reset();
+    for (int64_t base = begin; base < end; base += blockDim.x)
+    {
+        const int64_t i = base + threadIdx.x;
+        const bool ok = i < end;
+        const int ci = ok ? cloud_of(coff, num_clouds, (int)i) : c;
+        const bool other = ci != c && c >= 0;
+        if (__any_sync(full, other))
+        {
+            flush(other);
+            if (other)
+                reset();
+        }
+        if (ok)
+        {
+            c = ci;
+            const float x = p[i * 3 + 0], y = p[i * 3 + 1], z = p[i * 3 + 2], wi = w ? w[i] : 0.0f;
+            v[0] = fminf(v[0], x);
+            v[1] = fminf(v[1], y);
+            v[2] = fminf(v[2], z);
+            v[3] = fmaxf(v[3], x);
+            v[4] = fmaxf(v[4], y);
+            v[5] = fmaxf(v[5], z);
+            v[6] = fmaxf(v[6], wi);
+        }
     }
+    flush(true);
 }
 
 // Per cloud: the reference box in FP32 (same operations as the reference) and the Morton frame.
