@@ -316,36 +316,50 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
                         __syncwarp();
                     }
                     PG_LANE_T1(C, kLaneCycSearch, t0);
-                    // all lanes test up to four of their points at a time
+                    // All lanes test up to four of their points at a time; the next four are loaded meanwhile.
                     int rd = rr >= 0.0f ? 0 : nr;
                     unsigned mw = 0;
-                    for (;;)
-                    {
-                        int j[4];
-                        Cand cq[4];
+                    int jn[4];
+                    float4 qn[4];
+                    auto pull = [&]() {
 #pragma unroll
                         for (int u = 0; u < 4; ++u)
                         {
                             while (mw == 0u && rd < nr)
                                 mw = cmask[rd++];
-                            j[u] = -1;
+                            jn[u] = -1;
                             if (mw != 0u)
                             {
                                 const int b = __ffs(mw) - 1;
                                 mw &= mw - 1u;
-                                j[u] = leaf_first(m.lv[2 * (rd - 1) + (b >> 4)]) + (b & 15);
+                                jn[u] = leaf_first(m.lv[2 * (rd - 1) + (b >> 4)]) + (b & 15);
                             }
                         }
-                        if (!__any_sync(kFull, j[0] >= 0))
-                            break;
 #pragma unroll
                         for (int u = 0; u < 4; ++u)
-                            cq[u] = make_cand(C.s, A.pts[max(j[u], 0)], j[u]);
+                            qn[u] = A.pts[max(jn[u], 0)];
+                    };
+                    pull();
+                    while (__any_sync(kFull, jn[0] >= 0))
+                    {
+                        int j[4];
+                        float4 q4[4];
+                        Cand cq[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                        {
+                            j[u] = jn[u];
+                            q4[u] = qn[u];
+                        }
+                        pull();
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            cq[u] = make_cand(C.s, q4[u], j[u]);
                         const unsigned may = j[0] >= 0 ? C.may_cut4(cq) : 0u;
 #pragma unroll
                         for (int u = 0; u < 4; ++u)
                             if (j[u] >= 0 && ((may >> u) & 1u) &&
-                                !(!GUESS && shell == 0 && j[u] <= jK && lane_sq_dist(C.s, A.pts[j[u]]) == dK)) // (clipped before)
+                                !(!GUESS && shell == 0 && j[u] <= jK && lane_sq_dist(C.s, q4[u]) == dK)) // (clipped)
                             {
                                 if (nk < kLaneCut)
                                     cand[nk] = j[u];
