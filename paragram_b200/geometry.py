@@ -69,20 +69,26 @@ def face_areas(points: torch.Tensor, weights: Optional[torch.Tensor] = None, *, 
     NaN for a cell with more than ``capacity`` vertices (at most 256).
     """
     from . import _lib
+    from .cuda import build_with_stats
 
-    d, vx = cell_vertices(points, weights, capacity=capacity, knn=knn, leaf_size=leaf_size)
     points = _validate_points(points)
+    if weights is not None:
+        weights = _validate_weights(weights, points.shape[0], points.device)
+    (adjacency, offsets, status), out = build_with_stats(points, weights, knn=knn, leaf_size=leaf_size,
+                                                         vertices=capacity)
+    d = Diagram(adjacency=adjacency, offsets=offsets, status=status)
     n = int(points.shape[0])
     areas = torch.empty(max(d.adjacency.numel(), 1), dtype=torch.float32, device=points.device)
     if n > 0 and d.adjacency.numel() > 0:
         lib = _lib.load()
-        rel = vx["relative"]
-        # the library reads the exported float4 rows (x, y, z, bound)
-        v4 = torch.cat([rel, vx["bound"][..., None]], dim=2).contiguous()
+        # the exported float4 rows (x, y, z, bound), of which out["vertices"] is a view from their start
+        v4 = out["vertices"]
+        if v4.stride() != (4 * int(capacity), 4, 1):
+            raise RuntimeError("unexpected layout of the exported vertices")
         with torch.cuda.device(points.device):
-            rc = lib.pg_face_areas(n, int(capacity), v4.data_ptr(), vx["planes"].contiguous().data_ptr(),
-                                   vx["count"].contiguous().data_ptr(), points.data_ptr(), d.offsets.data_ptr(),
-                                   d.adjacency.data_ptr(), areas.data_ptr(),
+            rc = lib.pg_face_areas(n, int(capacity), v4.data_ptr(), out["vertex_planes"].contiguous().data_ptr(),
+                                   out["vertex_count"].contiguous().data_ptr(), points.data_ptr(),
+                                   d.offsets.data_ptr(), d.adjacency.data_ptr(), areas.data_ptr(),
                                    torch.cuda.current_stream(points.device).cuda_stream)
         if rc != 0:
             raise RuntimeError(_lib.last_error(lib))
