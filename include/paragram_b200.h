@@ -59,9 +59,10 @@ typedef struct pg_options
     int32_t num_chunks; /* reference: PARAGRAM_NUM_CHUNKS / PARAGRAM_MEM_FRAC chunk plan
                            (chunking.h:16-56). 0 = read the environment; > 0 = split the cell
                            pass into this many launches. Results do not depend on it. */
-    int32_t blocks_per_sm; /* register budget of the cell kernel: resident blocks of 8 warps per SM
-                              (2 or 3; 0 = default 2). No reference counterpart; chosen by the
-                              autotuner. Results do not depend on it. */
+    int32_t blocks_per_sm; /* register budget of the warp-per-cell kernel: resident blocks of 8 warps per SM
+                              (2 or 3; 0 = default 2). 3 also keeps a large build from the cell-per-lane
+                              pass. No reference counterpart; chosen by the autotuner. Results do not
+                              depend on it. */
     int32_t predicates;    /* 0 (default): FP32 side tests behind a rigorous error filter, undecided ones
                               re-evaluated in FP64 and exact expansions (exact results). 1: FP32 side
                               tests only, undecided ones taken by the sign of the FP32 value, as the

@@ -431,7 +431,7 @@ static int build_impl(int64_t n, int num_clouds, const int32_t *cloud_offsets, c
     // points. Batches are mostly surface clouds, whose cells it leaves to the warp-per-cell pass.
     const int64_t cells = ranged ? range_end - range_begin : n;
     cl.lanes = cells >= kLaneMinCells && num_clouds == 1 && leaf <= kDefaultLeaf && !cl.fp32_only &&
-               !opt.radius_out && !opt.work_out && opt.blocks_per_sm == 0;
+               !opt.radius_out && !opt.work_out && opt.blocks_per_sm != 3;
     int chunks = sync ? plan_chunks(n, opt.num_chunks) : std::max(opt.num_chunks, 1);
     int sms = device_sms();
     const int64_t rb = ranged ? range_begin : 0, re = ranged ? range_end : n;

@@ -41,7 +41,7 @@ constexpr int kBigWarps = 4;        // warps per block of the 256-slot tier (sta
 constexpr int kMidWarps = 4;        // warps per block of the 128-slot tier (13 KB of shared memory each)
 constexpr int kMidBlocksPerSM = 3;  // its resident blocks per SM (up to 170 registers per thread)
 #ifndef PG_LANE_V
-#define PG_LANE_V 48
+#define PG_LANE_V 42
 #endif
 #ifndef PG_LANE_WARM
 #define PG_LANE_WARM 16
@@ -49,7 +49,9 @@ constexpr int kMidBlocksPerSM = 3;  // its resident blocks per SM (up to 170 reg
 #ifndef PG_LANE_MIN
 #define PG_LANE_MIN 32768
 #endif
-constexpr int kLaneV = PG_LANE_V;       // vertex slots of a cell of the cell-per-lane pass
+// Vertex slots of a cell of the cell-per-lane pass: with 42 eight one-warp blocks fit in an SM's shared memory,
+// with 48 seven (2M clustered cells 38.6 against 41.0 ms), with 36 nine, but too many cells outgrow them (44.6).
+constexpr int kLaneV = PG_LANE_V;
 constexpr int kLaneWarm = PG_LANE_WARM; // nearest points that clip it first
 constexpr int64_t kLaneMinCells = PG_LANE_MIN; // smallest build of that pass
 constexpr int kMaxLeaf = 32;        // leaf size limit (one candidate per lane)

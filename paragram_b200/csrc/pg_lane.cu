@@ -16,17 +16,17 @@
 // kept for clipping; (4) in clipping every lane first looks for its next point that
 // cuts, then all clip. Lanes that search on their own (a traversal per lane, whether
 // left to diverge or scheduled step by step) ran at 4 to 10 active lanes: 45 and
-// 22 ms for 500,000 clustered cells, against 21 ms for a warp per cell and 12 here.
+// 22 ms for 500,000 clustered cells, against 21 ms for a warp per cell and 11 here.
 // Eight lanes per cell: 26 ms (instruction-cache misses between the steps).
 //
 // A cell that does not fit (more than kLaneV vertices or kLaneP planes at a time, a
 // reach that holds more than kLaneMarks points: cells at the hull, beside a far denser
 // region, or long cells of surface data) is listed for the warp-per-cell pass.
 //
-// Measured on one B200, first pass with its kNN query and listed cells: 5M clustered
-// points 214 -> 103 ms, 1M uniform power 43.6 -> 21.4 ms, jittered 128^3 power lattice
-// 87.5 -> 21.9 ms. Bound by latency: one warp per block, 7 blocks per SM (31 KB of shared
-// memory each), 33% of the issue slots used.
+// Measured on one B200, first pass with its kNN query and listed cells: 2M clustered
+// points 86 -> 38.6 ms, 500,000 21.0 -> 11.2 ms, 500,000 uniform power 21.8 -> 10.0 ms,
+// jittered 80^3 power lattice 21.4 -> 6.1 ms. Bound by latency: one warp per block, 8
+// blocks per SM (28 KB of shared memory each), a third of the issue slots used (with 7).
 #include <algorithm>
 
 #include "pg_kernels.cuh"
@@ -36,7 +36,7 @@ namespace pg
 {
 
 #ifndef PG_LANE_BLOCKS
-#define PG_LANE_BLOCKS 7
+#define PG_LANE_BLOCKS 8
 #endif
 #ifndef PG_LANE_SHELL
 #define PG_LANE_SHELL 2.5f
@@ -47,7 +47,7 @@ namespace pg
 #ifndef PG_LANE_MARKS
 #define PG_LANE_MARKS 96
 #endif
-constexpr int kLaneBlocks = PG_LANE_BLOCKS; // resident one-warp blocks per SM (31 KB of shared memory each)
+constexpr int kLaneBlocks = PG_LANE_BLOCKS; // resident one-warp blocks per SM (28 KB of shared memory each)
 // Squared radius of the first search over the last near point's. 500,000 clustered cells: 2.0 14.5, 2.5 13.8,
 // 3.0 14.8 ms (a smaller one leaves more cells to the second search, a larger one more points to test).
 constexpr float kLaneShell = PG_LANE_SHELL;

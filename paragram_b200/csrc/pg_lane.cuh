@@ -3,7 +3,7 @@
 // Shared memory is laid out [slot][lane], so that the lanes' accesses never share a bank
 // whatever slots they are at. A vertex takes 16 bytes, its plane triple in the low bits
 // of its error radius; planes are not stored but recomputed from their points, whose
-// loads L1 and L2 serve, so that 224 cells fit in an SM's shared memory.
+// loads L1 and L2 serve, so that 256 cells fit in an SM's shared memory.
 #pragma once
 
 #include "pg_clip.cuh"
