@@ -52,7 +52,7 @@ sys.path.insert(0, ROOT)
 import numpy as np  # noqa: E402
 
 MEASURED_PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
-PROFILE_SUMMARY = os.path.join(ROOT, "profiles", "k_cells_fast_clustered5m.txt")
+PROFILE_SUMMARY = os.path.join(ROOT, "profiles", "k_cells_lane_clustered5m.txt")
 
 WORKLOADS = {
     "clustered_voronoi_5m": dict(kind="clustered", n=5_000_000, weighted=False),
@@ -670,7 +670,7 @@ def run_gpu(args, spec, rank, world, local):
             "step_ms": [round(t, 2) for t in times],
             "config": config,
             "e2e": {"value": e2e_value, "unit": "Mcells/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
-            "roofline": _roofline(flops, nbytes, cell_s, csum, "k_cells_fast (cell pass)",
+            "roofline": _roofline(flops, nbytes, cell_s, csum, "k_cells_lane (cell pass)",
                                   read_traffic_per_launch() if args.workload == "clustered_voronoi_5m" else None),
             "cpu_baseline": _cpu_baseline(args, world, pts, w, n),
             "clocks": csum,
@@ -770,7 +770,7 @@ def run_lattice_gpu(args, spec, rank, world, local, dev):
                        "status_counts": np.bincount(d.status.cpu().numpy(), minlength=6)[:6].tolist(),
                        "phases_ms": {k: round(prof[k], 3) for k in ("lbvh_ms", "cells_ms", "deferred_ms", "csr_ms")}},
             "e2e": {"value": e2e_value, "unit": "Mcells/s", "h2d_bytes_per_step": n * 16, "d2h_bytes_per_step": d2h},
-            "roofline": _roofline(flops, nbytes, cell_s, csum, "k_cells_fast (cell pass)", None),
+            "roofline": _roofline(flops, nbytes, cell_s, csum, "k_cells_lane (cell pass)", None),
             "cpu_baseline": _cpu_baseline(args, world, pts, w, n),
             "clocks": csum,
             "gpu_launches": int(prof["launches"]) * args.steps,
@@ -933,7 +933,7 @@ def run_moving_gpu(args, spec, rank, world, local, dev):
                        "phases_ms": {k_: round(prof[k_], 3) for k_ in ("lbvh_ms", "cells_ms", "deferred_ms",
                                                                        "csr_ms")}},
             "e2e": {"value": e2e_value, "unit": "Mcells/s", "h2d_bytes_per_step": n * 12, "d2h_bytes_per_step": d2h},
-            "roofline": _roofline(flops, nbytes, cell_s, csum, "k_cells_fast (cell pass)", None),
+            "roofline": _roofline(flops, nbytes, cell_s, csum, "k_cells_lane (cell pass)", None),
             "cpu_baseline": _cpu_baseline(args, world, pts, None, n),
             "clocks": csum,
             "gpu_launches": int(prof["launches"]) * args.steps,
