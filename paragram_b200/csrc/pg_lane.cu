@@ -6,7 +6,7 @@
 // the cells are the same; what differs is who does the work. A warp per cell issues
 // every step of a cell's search once per cell (28,900 warp instructions for a cell of
 // about 27 vertices, 21.8 of 32 lanes active); 32 cells per warp, kept in step, share
-// them: 8,100 for 32 cells' steps per cell.
+// them: 6,400 per cell.
 //
 // What keeps the lanes in step: (1) a cell is first clipped by its kLaneWarm nearest
 // points (k_knn), nearly all of which cut it; (2) the points that can still
@@ -26,7 +26,7 @@
 // Measured on one B200, first pass with its kNN query and listed cells: 2M clustered
 // points 86 -> 38.6 ms, 500,000 21.0 -> 11.2 ms, 500,000 uniform power 21.8 -> 10.0 ms,
 // jittered 80^3 power lattice 21.4 -> 6.1 ms. Bound by latency: one warp per block, 8
-// blocks per SM (28 KB of shared memory each), a third of the issue slots used (with 7).
+// blocks per SM (28 KB of shared memory each), 38% of the issue slots used.
 #include <algorithm>
 
 #include "pg_kernels.cuh"
