@@ -55,7 +55,7 @@ size_t workspace_layout(int64_t n, int num_clouds, char *base, Workspace *ws)
         return p;
     };
     size_t N = (size_t)std::max<int64_t>(n, 1);
-    int blocks = sort_blocks((int64_t)N);
+    int blocks = sort_blocks_upto((int64_t)N);
     size_t hist_elems = (size_t)256 * blocks + 1;
     size_t scan_elems = scan_tmp_elems((int64_t)std::max(hist_elems, N + 1));
     Workspace w;

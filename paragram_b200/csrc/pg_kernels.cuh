@@ -18,7 +18,7 @@ size_t scan_tmp_elems(int64_t n);
 void exclusive_scan(const uint32_t *in, uint32_t *out, int64_t n, uint32_t *tmp, cudaStream_t st);
 
 // pg_lbvh.cu
-int sort_blocks(int64_t n);
+int sort_blocks_upto(int64_t n); // sizes the sort's histograms
 void lbvh_build(const Workspace &ws, int64_t n, int num_clouds, const float *points, const float *weights,
                 int leaf_size, cudaStream_t st);
 

@@ -30,7 +30,11 @@ constexpr int kSortSteps = 16, kSortStepsSmall = 4;
 constexpr int64_t kSortSmall = 600000;
 static int sort_tile(int64_t n) { return kSortThreads * (n < kSortSmall ? kSortStepsSmall : kSortSteps); }
 
-int sort_blocks(int64_t n) { return (int)((n + sort_tile(n) - 1) / sort_tile(n)); }
+static int sort_blocks(int64_t n) { return (int)((n + sort_tile(n) - 1) / sort_tile(n)); }
+
+// Blocks whose histograms a workspace for n keys holds: no fewer than any smaller sort takes (599,999 keys are
+// 586 small tiles, 600,000 only 147 large ones), so that a workspace also serves every smaller build.
+int sort_blocks_upto(int64_t n) { return std::max(sort_blocks(n), sort_blocks(std::min(n, kSortSmall - 1))); }
 
 // Up to kSortOne keys are sorted by one block in shared memory (a launch instead of 8 passes of 3).
 constexpr int kSortOne = 4096;

@@ -41,6 +41,18 @@ def test_workspace_size(lib):
     assert lib.pg_workspace_size(1 << 26, ctypes.byref(n)) == -1
 
 
+@pytest.mark.parametrize("around", [4096, 600_000, 601_088, 4_000_000])
+@pytest.mark.parametrize("clouds", [1, 5])
+def test_workspace_size_never_decreases(lib, around, clouds):
+    """A workspace sized for a maximum serves every smaller build."""
+    size, last = ctypes.c_size_t(0), 0
+    for n in range(around - 1500, around + 1500):
+        assert (lib.pg_workspace_size(n, ctypes.byref(size)) if clouds == 1 else
+                lib.pg_batch_workspace_size(n, clouds, ctypes.byref(size))) == 0
+        assert size.value >= last, n
+        last = size.value
+
+
 def _build(lib, n, points=1, weights=None, guesses=None, goff=None, ws=256, ws_bytes=1 << 40, offsets=256,
            status=256, options=None):
     from paragram_b200 import _lib
