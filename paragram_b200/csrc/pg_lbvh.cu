@@ -58,11 +58,11 @@ __global__ void __launch_bounds__(256) k_bounds(const float *__restrict__ p, con
     const int64_t per = ((n + gridDim.x - 1) / gridDim.x + blockDim.x - 1) / blockDim.x * blockDim.x;
     const int64_t begin = (int64_t)blockIdx.x * per, end = min(n, begin + per);
     int c = -1; // the cloud of v
-    float v[7];
+    int v[7];   // as order-preserving integers: NaN, above infinity, is kept (fminf and fmaxf would drop it)
     auto reset = [&]() {
 #pragma unroll
         for (int k = 0; k < 7; ++k)
-            v[k] = k < 3 ? INFINITY : -INFINITY;
+            v[k] = float_to_ordered(k < 3 ? INFINITY : -INFINITY);
     };
     auto flush = [&](bool mine_too) {
         unsigned todo = __ballot_sync(full, mine_too && c >= 0);
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(256) k_bounds(const float *__restrict__ p, con
 #pragma unroll
             for (int k = 0; k < 7; ++k)
             {
-                const int key = float_to_ordered(mine ? v[k] : (k < 3 ? INFINITY : -INFINITY));
+                const int key = mine ? v[k] : float_to_ordered(k < 3 ? INFINITY : -INFINITY);
                 const int r = k < 3 ? __reduce_min_sync(full, key) : __reduce_max_sync(full, key);
                 if ((int)(threadIdx.x & 31) == leader)
                 {
@@ -103,14 +103,14 @@ __global__ void __launch_bounds__(256) k_bounds(const float *__restrict__ p, con
         if (ok)
         {
             c = ci;
-            const float x = p[i * 3 + 0], y = p[i * 3 + 1], z = p[i * 3 + 2], wi = w ? w[i] : 0.0f;
-            v[0] = fminf(v[0], x);
-            v[1] = fminf(v[1], y);
-            v[2] = fminf(v[2], z);
-            v[3] = fmaxf(v[3], x);
-            v[4] = fmaxf(v[4], y);
-            v[5] = fmaxf(v[5], z);
-            v[6] = fmaxf(v[6], wi);
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+            {
+                const int x = float_to_ordered(p[i * 3 + k]);
+                v[k] = min(v[k], x);
+                v[3 + k] = max(v[3 + k], x);
+            }
+            v[6] = max(v[6], float_to_ordered(w ? w[i] : 0.0f));
         }
     }
     flush(true);

@@ -131,3 +131,31 @@ def test_lbvh_duplicates(dev):
     pts = np.repeat(base, 5, axis=0)
     spts, order, rec, roots = _build(pts, None, [0, len(pts)], -1, dev)
     _check_tree(pts, None, [0, len(pts)], -1, spts, order, rec, roots)
+
+
+@pytest.mark.parametrize("n", [40, 5000])
+def test_bounds_keep_non_finite_values(dev, n):
+    """A NaN (above infinity in the bounds' order) or infinite coordinate or weight stays in the cloud's
+    bounds. A range build without cells makes the tree alone."""
+    from paragram_b200 import _lib
+
+    lib = _lib.load()
+    rng = np.random.default_rng(8)
+    pts, w = rng.random((n, 3), dtype=np.float32), rng.random(n, dtype=np.float32)
+    pts[n // 3, 0], pts[n // 2, 1], w[n - 1] = np.nan, np.inf, np.nan
+    p, t = torch.from_numpy(pts).to(dev), torch.from_numpy(w).to(dev)
+    size = ctypes.c_size_t(0)
+    assert lib.pg_workspace_size(n, ctypes.byref(size)) == 0
+    ws = torch.empty(size.value, dtype=torch.uint8, device=dev)
+    status = torch.empty(n, dtype=torch.int32, device=dev)
+    opt = _lib.PgOptions(8, -1, 0, 0, 0)
+    assert lib.pg_build_range(n, p.data_ptr(), t.data_ptr(), ctypes.byref(opt), ws.data_ptr(), size.value, 0, 0,
+                              status.data_ptr(), torch.cuda.current_stream(dev).cuda_stream) == 0
+    out = (ctypes.c_int64 * 5)()
+    assert lib.pg_workspace_tree(n, 1, out, 5) == 0
+    box = ws.cpu().numpy()[out[4]:out[4] + 28].view(np.float32)
+    finite = np.isfinite(pts)
+    lo = [np.float32(pts[finite[:, k], k].min()) - np.float32(1) - np.float32(1e-5) for k in range(3)]
+    hi = np.float32(pts[finite[:, 2], 2].max()) + np.float32(1) + np.float32(1e-5)
+    assert np.array_equal(box[:3], np.array(lo, np.float32)) and box[5] == hi
+    assert np.isnan(box[3]) and np.isinf(box[4]) and np.isnan(box[6])
