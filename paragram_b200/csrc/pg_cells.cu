@@ -83,7 +83,7 @@ template <int CAP, int STACK> struct CellMem
     float cap;  // search radius of the current pass (learned / given; +inf without one)
     float done; // search radius of the finished first pass (-inf during the first pass)
     unsigned et[CAP * CAP / 32];       // edge table of the clip in progress (all zero between clips)
-    typename std::conditional<(CAP <= 256), unsigned char, unsigned short>::type rl[CAP]; // its removed slots, by rank
+    typename std::conditional<(CAP <= 256), unsigned char, unsigned short>::type rl[CAP]; // its removed, then free slots
 };
 
 // Clear a warp's edge table (once, before its first clip).
@@ -305,10 +305,12 @@ enum ClipResult : int
 // tested, listed by ballots), then the r-th boundary edge (in the r-th removed slot, then in free ones).
 // Listing edges and searching slots word by word instead cost the larger tiers, whose time is the chain of
 // their slowest cells, 39.7 ms in the 256-slot tier of 24 surface clouds (25.7 so) and 8.0 in the 128-slot
-// tier (7.0); the 64-slot pass takes 21.8 against 21.2 ms there.
+// tier (7.0). The free slots are listed behind the removed ones: a lane that looked for its own, one set bit
+// after the other, cost 7% in the 64-slot pass (24 uniform clouds 17.9 ms, 16.7 so; 200,000 points with FP32
+// predicates 9.47 and 8.79 ms).
 template <int CAP, int STACK>
 __device__ __forceinline__ int clip(CellMem<CAP, STACK> &m, WarpState<CAP> &ws, const Cand &q, const CellArgs &A,
-                                           int lane)
+                                    int lane)
 {
     constexpr int W = CAP / 32;
     const unsigned lt = (1u << lane) - 1u;
@@ -413,7 +415,18 @@ __device__ __forceinline__ int clip(CellMem<CAP, STACK> &m, WarpState<CAP> &ws, 
         }
     if (nvalid - nr + nb > CAP)
         return kClipDefer;
-    __syncwarp(); // all reads of removed triangles are done
+    // the boundary edges beyond the removed slots go to the free ones, in order
+    int at = nr;
+#pragma unroll(CAP > 256 ? 1 : CAP / 32)
+    for (int k = 0; k < W; ++k)
+    {
+        const unsigned f = ~ws.valid[k];
+        const int r = at + __popc(f & lt);
+        if (((f >> lane) & 1u) && r < nb)
+            m.rl[r] = k * 32 + lane;
+        at += __popc(f);
+    }
+    __syncwarp(); // the slots; all reads of removed triangles are done
     const float4 pP = m.pl[P];
     const float eP = m.pe[P];
     for (int r0 = 0; r0 < nb; r0 += 32)
@@ -429,26 +442,7 @@ __device__ __forceinline__ int clip(CellMem<CAP, STACK> &m, WarpState<CAP> &ws, 
             const unsigned xy = m.eb[r];
             x = xy & 0xFFFFu;
             y = xy >> 16;
-            if (r < nr)
-                slot = m.rl[r];
-            else
-            {
-                int u = r - nr; // the u-th free slot
-                slot = -1;
-#pragma unroll(CAP > 256 ? 1 : CAP / 32)
-                for (int k = 0; k < W; ++k)
-                {
-                    unsigned f = ~ws.valid[k];
-                    const int c = __popc(f);
-                    if (slot < 0 && u < c)
-                    {
-                        for (int v = 0; v < u; ++v)
-                            f &= f - 1u;
-                        slot = k * 32 + __ffs(f) - 1;
-                    }
-                    u -= c;
-                }
-            }
+            slot = m.rl[r];
             X = make_vertex(pP, eP, m.pl[x], m.pe[x], m.pl[y], m.pe[y], vr);
             ill = !(X.w <= kVertex64Rel * (fabsf(X.x) + fabsf(X.y) + fabsf(X.z)));
         }
