@@ -61,8 +61,9 @@ typedef struct pg_options
                            pass into this many launches. Results do not depend on it. */
     int32_t blocks_per_sm; /* register budget of the warp-per-cell kernel: resident blocks of 8 warps per SM
                               (2 or 3; 0 = default 2). 3 also keeps a large build from the cell-per-lane
-                              pass. No reference counterpart; chosen by the autotuner. Results do not
-                              depend on it. */
+                              pass. No reference counterpart; chosen by the autotuner. Rows, offsets and
+                              statuses do not depend on it; exported vertices and integrals agree within
+                              their error bounds, the vertices of a cell in any order. */
     int32_t predicates;    /* 0 (default): FP32 side tests behind a rigorous error filter, undecided ones
                               re-evaluated in FP64 and exact expansions (exact results). 1: FP32 side
                               tests only, undecided ones taken by the sign of the FP32 value, as the
@@ -231,7 +232,9 @@ int pg_knn(int64_t num_points, const float *points, int32_t k, void *workspace, 
  * out[0] kernel launches, out[1] LBVH ms, out[2] cell pass ms, out[3] deferred-cell
  * pass ms, out[4] CSR count + scan ms, out[5] deferred cells, out[6] cell-pass chunks,
  * out[7] deferred cells rebuilt with 256 slots, out[8] with 512 slots, out[9] cells a
- * learned model routed past the first pass (pg_model.route_degree).
+ * learned model routed past the first pass (pg_model.route_degree), out[10] cells that the
+ * cell-per-lane pass took (0: the warp-per-cell pass built all), out[11] those of them that it
+ * left to the warp-per-cell pass.
  * The times are recorded only when options->debug != 0 (CUDA events on the stream).
  * No reference counterpart (the reference prints timings with debug=True,
  * voronoi_ultra.cu:196-219, 368-373). */

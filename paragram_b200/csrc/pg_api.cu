@@ -22,7 +22,7 @@ namespace pg
 
 static thread_local std::string g_last_error;
 thread_local long long g_launches = 0;
-static thread_local double g_profile[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+static thread_local double g_profile[12] = {};
 
 static int fail(int code, const std::string &msg)
 {
@@ -426,24 +426,31 @@ static int build_impl(int64_t n, int num_clouds, const int32_t *cloud_offsets, c
     }
     // One cell per lane (pg_lane.cu) where that fills the GPU and no per-cell diagnostics are asked for: a lane
     // takes about 0.9 ms for its cell however few there are, so below kLaneMinCells the warp-per-cell pass is
-    // faster (uniform points: 24,000 1.60 against 1.61 ms, 32,000 2.22 against 1.98, 96,000 5.19 against 3.51;
-    // clustered: 48,000 3.17 against 3.34, 64,000 3.80 against 3.60). Its leaf scans take leaves of up to 16
-    // points. Batches are mostly surface clouds, whose cells it leaves to the warp-per-cell pass.
+    // faster (uniform points: 24,000 1.60 against 1.61 ms, 33,000 2.00 against 1.73, 100,000 5.13 against 3.32).
+    // From there on a survey of the points decides (LaneChoice). Its leaf scans take leaves of up to 16 points;
+    // batches of several clouds keep the warp-per-cell pass.
     const int64_t cells = ranged ? range_end - range_begin : n;
     cl.lanes = cells >= kLaneMinCells && num_clouds == 1 && leaf <= kDefaultLeaf && !cl.fp32_only &&
                !opt.radius_out && !opt.work_out && opt.blocks_per_sm != 3;
+    cl.choice = LaneChoice{ws.counters, 1, cells < kLaneAnyCells};
+    if (cl.lanes)
+        cl.choice.groups = lane_survey_launch(ws, n, st);
     int chunks = sync ? plan_chunks(n, opt.num_chunks) : std::max(opt.num_chunks, 1);
     int sms = device_sms();
     const int64_t rb = ranged ? range_begin : 0, re = ranged ? range_end : n;
-    int64_t per = (re - rb + chunks - 1) / chunks;
+    // chunks end at multiples of 32 of the curve order: a group of the cell-per-lane pass lies within one
+    const int64_t r0 = rb & ~(int64_t)31;
+    const int64_t per = ((re - r0 + chunks - 1) / chunks + 31) & ~(int64_t)31;
     for (int c = 0; c < chunks; ++c)
     {
-        cl.cell_begin = rb + (int64_t)c * per;
-        cl.cell_end = std::min<int64_t>(re, cl.cell_begin + per);
+        cl.cell_begin = std::max<int64_t>(rb, r0 + (int64_t)c * per);
+        cl.cell_end = std::min<int64_t>(re, r0 + (int64_t)(c + 1) * per);
         if (cl.cell_begin >= cl.cell_end)
             break;
         cells_launch(ws, cl, status, sms, st);
     }
+    cl.cell_begin = rb;
+    cl.cell_end = re;
     if (cl.lanes)
         cells_list_launch(ws, cl, status, sms, st);
     if (timing)
@@ -462,13 +469,13 @@ static int build_impl(int64_t n, int num_clouds, const int32_t *cloud_offsets, c
         cudaError_t e = cudaGetLastError();
         return e == cudaSuccess ? PG_OK : fail(PG_ERR_CUDA, std::string("CUDA error: ") + cudaGetErrorString(e));
     }
-    int host[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    int host[16] = {};
     int64_t edges = 0;
     {
         uint32_t e32 = 0;
         if (!ranged)
             cudaMemcpyAsync(&e32, offsets + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(host, ws.counters, 8 * sizeof(int), cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(host, ws.counters, 16 * sizeof(int), cudaMemcpyDeviceToHost, st);
         cudaError_t e = cudaStreamSynchronize(st);
         if (e != cudaSuccess)
             return fail(PG_ERR_CUDA, std::string("CUDA error: ") + cudaGetErrorString(e));
@@ -501,6 +508,12 @@ static int build_impl(int64_t n, int num_clouds, const int32_t *cloud_offsets, c
     g_profile[7] = (double)host[5];                                 // rebuilt with 256 slots
     g_profile[8] = (double)std::min(host[4], kHugeSlabs);           // rebuilt with 512 slots
     g_profile[9] = (double)std::min<int64_t>(host[7], route_cap(n)); // routed past the first pass
+    cl.choice.counters = host;
+    if (cl.lanes && !cl.choice.declined())
+    {
+        g_profile[10] = (double)cells;              // taken by the cell-per-lane pass
+        g_profile[11] = (double)host[kCountListed]; // of them left to the warp-per-cell pass
+    }
     int rc = check_counters(host, n);
     if (rc != PG_OK)
         return rc;
@@ -704,7 +717,7 @@ int pg_last_profile(double *out, int32_t count)
 {
     if (!out || count < 0)
         return pg::fail(PG_ERR_INVALID, "bad arguments");
-    for (int i = 0; i < count && i < 10; ++i)
+    for (int i = 0; i < count && i < 12; ++i)
         out[i] = pg::g_profile[i];
     return PG_OK;
 }

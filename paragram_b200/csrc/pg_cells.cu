@@ -1393,9 +1393,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, MINB) k_cells_fast(CellAr
 }
 
 
-// The cells that the cell-per-lane pass listed (their number in counters[8]), as the first pass builds them.
+// The cells that the cell-per-lane pass listed, or all of the build's where it was declined, as the first pass
+// builds them.
 // A body of its own: the first pass's code is kept as it is (a branch on the cell's source in its loop made
 // builds with a geometry export 5% slower, from the changed layout of the code alone).
+template <bool GUESS, bool HINT>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, kMinBlocksLo) k_cells_list(CellArgs A)
 {
     __shared__ CellMem<kCapFast, kStackFast> mem[kWarpsPerBlock];
@@ -1405,7 +1407,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kMinBlocksLo) k_cells_lis
     if (lane < kNumStats)
         m.cnt[lane] = 0;
     clear_edges(m, lane);
-    const int count = A.counters[8];
+    const bool all = A.choice.declined();
+    const int count = all ? (int)(A.end - A.begin) : A.counters[kCountListed];
     for (;;)
     {
         int t = 0;
@@ -1414,8 +1417,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kMinBlocksLo) k_cells_lis
         t = __shfl_sync(kFull, t, 0);
         if (t >= count)
             break;
-        const int i = A.list[t];
-        process_cell<kCapFast, kStackFast, false, false>(m, ws, i, A, lane);
+        const int i = all ? (int)A.begin + t : A.list[t];
+        // (a cell the learned model routed to the 128-slot tier, as in the first pass)
+        if (HINT && A.hint != nullptr && A.hint[i] < 0.0f)
+            continue;
+        process_cell<kCapFast, kStackFast, GUESS, HINT>(m, ws, i, A, lane);
         write_diagnostics(m, ws, A, lane);
         if (__any_sync(kFull, ws.flags & kFlagError))
         {
@@ -1570,6 +1576,7 @@ static CellArgs make_args(const Workspace &ws, const CellLaunch &cl)
     A.begin = cl.cell_begin;
     A.end = cl.cell_end;
     A.list = nullptr;
+    A.choice = cl.choice;
     A.big_cap = 0;
     A.huge_slabs = (char *)ws.huge_slabs;
     A.radius_out = cl.radius_out;
@@ -1594,7 +1601,8 @@ void cells_launch(const Workspace &ws, const CellLaunch &cl, int *status, int nu
     if (cl.lanes)
     {
         if (!cl.guesses)
-            knn_rows_launch(ws, cl.num_clouds, cl.cell_begin, cl.cell_end, st);
+            knn_rows_launch(ws, cl.num_clouds, cl.cell_begin & ~(int64_t)31, std::min(cl.n, (cl.cell_end + 31) & ~(int64_t)31),
+                            cl.choice, st);
         lane_launch(A, ws.flags, num_sms, st);
         return;
     }
@@ -1640,8 +1648,8 @@ void cells_launch(const Workspace &ws, const CellLaunch &cl, int *status, int nu
     kern<<<(unsigned)grid, kWarpsPerBlock * 32, 0, st>>>(A);
 }
 
-// The cells that the cell-per-lane pass listed (in the refit's arrival counters, free by now); their number
-// stays on the device: a fixed grid reads it.
+// The cells that the cell-per-lane pass listed (in the refit's arrival counters, free by now), or all of
+// [cell_begin, cell_end); which is known on the device: a fixed grid reads it.
 void cells_list_launch(const Workspace &ws, const CellLaunch &cl, int *status, int num_sms, cudaStream_t st)
 {
     CellArgs A = make_args(ws, cl);
@@ -1650,7 +1658,9 @@ void cells_list_launch(const Workspace &ws, const CellLaunch &cl, int *status, i
     A.list = ws.flags;
     cudaMemsetAsync(ws.counters, 0, sizeof(int), st);
     ++g_launches;
-    k_cells_list<<<(unsigned)(num_sms * kMinBlocksLo), kWarpsPerBlock * 32, 0, st>>>(A);
+    void (*kern)(CellArgs) = cl.guesses ? (cl.use_hint ? k_cells_list<true, true> : k_cells_list<true, false>)
+                                        : (cl.use_hint ? k_cells_list<false, true> : k_cells_list<false, false>);
+    kern<<<(unsigned)(num_sms * kMinBlocksLo), kWarpsPerBlock * 32, 0, st>>>(A);
 }
 
 // The deferred counts stay on the device: fixed grids read them. The middle

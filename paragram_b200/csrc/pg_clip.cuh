@@ -44,7 +44,8 @@ struct CellArgs
     int *counters;
     unsigned long long *stats;
     int64_t begin, end;
-    const int *list; // cells that the cell-per-lane pass left (sorted slots; their number in counters[8])
+    const int *list; // cells that the cell-per-lane pass left (sorted slots; their number in counters[kCountListed])
+    LaneChoice choice;
     int64_t big_cap;
     char *huge_slabs;
     float *radius_out; // optional per-cell diagnostics (original ids)

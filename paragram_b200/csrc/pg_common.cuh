@@ -54,10 +54,46 @@ constexpr int kMidBlocksPerSM = 3;  // its resident blocks per SM (up to 170 reg
 constexpr int kLaneV = PG_LANE_V;
 constexpr int kLaneWarm = PG_LANE_WARM; // nearest points that clip it first
 constexpr int64_t kLaneMinCells = PG_LANE_MIN; // smallest build of that pass
+// entries of the workspace's counters that the cell-per-lane pass uses: the cells it listed and, over the groups
+// that the survey sampled, the flat ones, the sum of their levels and of the levels' squares
+constexpr int kCountListed = 8, kCountFlat = 9, kCountLevel = 10, kCountLevelSq = 11;
 constexpr int kMaxLeaf = 32;        // leaf size limit (one candidate per lane)
 constexpr int kDefaultLeaf = 16;
 constexpr int kWindow = 16;         // optional warm start: sorted neighbours i-16 .. i+16
 constexpr uint32_t kBigFlag = 0x40000000u; // deg[] flag: row lives in the deferred-row area
+
+// Whether the cell-per-lane pass takes a build, from a survey of its points (k_lane_survey): a fixed sample of
+// the groups of 32 consecutive points of the curve, so that the choice, and with it every bit of a cell's export,
+// does not depend on the order in which anything runs. Known on the device only: the pass's kernels return at
+// once where it declines, and k_cells_list takes all cells.
+//
+// Flat groups: surface data, long cells whose reach holds too many points. A share of 0.2 to 0.4 up to 100,000
+// points of a surface cloud (58 to 66% of the cells would be listed: warp-per-cell pass 7.97 ms, cell-per-lane pass
+// 8.22 at 33,000 points; 15.5 and 16.0 at 100,000), 0.07 at 300,000 (43%; 31.4 and 30.9), 0.005 in clustered
+// volumes, 0 in uniform ones.
+//
+// Levels: in a build that the pass finishes in one or two waves, cells beside a far denser region are listed, and
+// the pass over the list takes as long as the slowest of them. Variance of the levels 2 to 3 in uniform points
+// (warp-per-cell pass 2.28 ms, cell-per-lane 2.11 at 40,000), 4.2 in 64 Gaussians of similar widths (2.18, 2.20),
+// 4.9 in 500 narrow ones (2.47, 3.03), 14 to 21 with widths from 0.005 to 0.1 (2.50, 2.80 at 40,000; 3.09, 3.14 at
+// 56,000; 3.24, 3.27 at 60,000; 4.02, 3.70 at 80,000).
+constexpr int kSurveyGroups = 512;
+constexpr int kLaneFlatShare = 10;         // declined above one flat group in ten
+constexpr int kLaneLevelVar2 = 9;          // declined below kLaneAnyCells above half this variance of the levels
+constexpr int64_t kLaneAnyCells = 60000;
+struct LaneChoice
+{
+    const int *counters; // the workspace's
+    int groups;          // groups sampled
+    int few;             // the build has fewer than kLaneAnyCells cells
+
+    __host__ __device__ bool declined() const
+    {
+        const int64_t flat = counters[kCountFlat], sum = counters[kCountLevel], sq = counters[kCountLevelSq];
+        return flat * kLaneFlatShare > groups ||
+               (few && 2 * (sq * groups - sum * sum) > (int64_t)kLaneLevelVar2 * groups * groups);
+    }
+};
 
 // statistics counters (uint64 each) in the workspace
 enum Stat : int

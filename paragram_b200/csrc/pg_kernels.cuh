@@ -45,6 +45,7 @@ struct CellLaunch
     int use_hint;      // the workspace holds a search radius per sorted slot
     int fp32_only;     // side tests in FP32 only (no escalation; not exact)
     int lanes;         // one cell per lane (pg_lane.cu), then cells_list_launch for those that do not fit
+    LaneChoice choice; // whether that pass takes the build (known on the device)
 };
 void cells_list_launch(const Workspace &ws, const CellLaunch &cl, int *status, int num_sms, cudaStream_t st);
 void cells_launch(const Workspace &ws, const CellLaunch &cl, int *status, int num_sms, cudaStream_t st);
@@ -52,11 +53,13 @@ void cells_big_launch(const Workspace &ws, const CellLaunch &cl, int *status, in
 
 // pg_lane.cu
 struct CellArgs;
+int lane_survey_launch(const Workspace &ws, int64_t n, cudaStream_t st); // returns the number of groups sampled
 void lane_launch(const CellArgs &A, int *list, int num_sms, cudaStream_t st);
 
 // pg_knn.cu: the kLaneWarm nearest other points (sorted slots, nearest first, -1: none) of the
-// sorted slots [begin, end), into the cells' rows
-void knn_rows_launch(const Workspace &ws, int num_clouds, int64_t begin, int64_t end, cudaStream_t st);
+// sorted slots [begin, end), into the cells' rows (nothing where the choice declines the pass)
+void knn_rows_launch(const Workspace &ws, int num_clouds, int64_t begin, int64_t end, const LaneChoice &choice,
+                     cudaStream_t st);
 
 // pg_mlp.cu
 void features_launch(const Workspace &ws, int64_t n, int num_clouds, float *out, cudaStream_t st);

@@ -61,8 +61,10 @@ __global__ void __launch_bounds__(128) k_knn(int64_t begin, int64_t end, const f
                                              const int *__restrict__ rparent, const int *__restrict__ pleaf,
                                              const int *__restrict__ cloud_off, int num_clouds,
                                              const int *__restrict__ cloud_root, int *__restrict__ out, int k,
-                                             int *err)
+                                             int *err, LaneChoice choice)
 {
+    if (ROWS && choice.declined())
+        return;
     const int64_t ii = begin + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool alive = ii < end;
     const int i = (int)(alive ? ii : end - 1);
@@ -171,14 +173,15 @@ __global__ void __launch_bounds__(128) k_knn(int64_t begin, int64_t end, const f
             o[t] = ROWS && full ? -2 : (best[t] == ~0ull ? -1 : (int)(unsigned)best[t]);
 }
 
-void knn_rows_launch(const Workspace &ws, int num_clouds, int64_t begin, int64_t end, cudaStream_t st)
+void knn_rows_launch(const Workspace &ws, int num_clouds, int64_t begin, int64_t end, const LaneChoice &choice,
+                     cudaStream_t st)
 {
     if (end <= begin)
         return;
     ++g_launches;
     k_knn<kLaneWarm, true><<<(unsigned)((end - begin + 127) / 128), 128, 0, st>>>(
         begin, end, ws.pts, ws.oid, ws.records, ws.rparent, ws.pleaf, ws.cloud_off, num_clouds, ws.cloud_root,
-        ws.rows, kLaneWarm, nullptr);
+        ws.rows, kLaneWarm, nullptr, choice);
 }
 
 } // namespace pg
@@ -213,7 +216,8 @@ extern "C" int pg_knn(int64_t num_points, const float *points, int32_t k, void *
     auto run = [&](auto kern) {
         kern<<<(unsigned)((num_points + 127) / 128), 128, 0, st>>>(0, num_points, ws.pts, ws.oid, ws.records,
                                                                    ws.rparent, ws.pleaf, ws.cloud_off, 1,
-                                                                   ws.cloud_root, neighbours, k, &ws.counters[2]);
+                                                                   ws.cloud_root, neighbours, k, &ws.counters[2],
+                                                                   LaneChoice{});
     };
     if (k <= 2)
         run(k_knn<2, false>);

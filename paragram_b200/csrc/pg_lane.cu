@@ -19,7 +19,8 @@
 // 22 ms for 500,000 clustered cells, against 21 ms for a warp per cell and 11 here.
 // Eight lanes per cell: 26 ms (instruction-cache misses between the steps).
 //
-// A cell that does not fit (more than kLaneV vertices or kLaneP planes at a time, a
+// Builds whose points would mostly be listed are declined as a whole (LaneChoice, pg_common.cuh). A cell that
+// does not fit (more than kLaneV vertices or kLaneP planes at a time, a
 // reach that holds more than kLaneMarks points: cells at the hull, beside a far denser
 // region, or long cells of surface data) is listed for the warp-per-cell pass.
 //
@@ -52,7 +53,6 @@ constexpr int kLaneBlocks = PG_LANE_BLOCKS; // resident one-warp blocks per SM (
 // 3.0 14.8 ms (a smaller one leaves more cells to the second search, a larger one more points to test).
 constexpr float kLaneShell = PG_LANE_SHELL;
 constexpr float kLaneFar = PG_LANE_FAR;     // the largest that a cell may need after it (beyond: listed)
-constexpr int kLaneTrial = 128;             // warps' worth of cells before their outcome decides about the rest
 constexpr int kLaneMarks = PG_LANE_MARKS;   // points of a search within a cell's reach
 
 // Optional per-phase SM cycle counters, as in pg_cells.cu (compile with -DPG_PHASE_CYCLES): the clips by the
@@ -87,6 +87,8 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
 {
     __shared__ LaneMem m;
     const int lane = threadIdx.x;
+    if (A.choice.declined())
+        return; // every cell is left to k_cells_list
     LaneCell C(m, A, lane);
     unsigned cmask[kLaneLeaves / 2];
     int cand[kLaneCut];
@@ -96,35 +98,15 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
         if (lane == 0)
             g = atomicAdd(&A.counters[0], 1);
         g = __shfl_sync(kFull, g, 0);
-        const int64_t gb = A.begin + (int64_t)g * 32;
+        const int64_t gb = (A.begin & ~(int64_t)31) + (int64_t)g * 32;
         if (gb >= A.end)
             break;
-        bool act = gb + lane < A.end;
-        {
-            // Where most cells so far had to be listed (surface data: long cells whose reach holds far too many
-            // points), the rest is listed at once. A cell costs 18 ns here against 45 to 70 ns in the
-            // warp-per-cell pass, so two in three have to succeed to pay for the rest.
-            int at = -1;
-            if (lane == 0)
-            {
-                const int done = __ldcg(&A.counters[9]), listed = __ldcg(&A.counters[8]);
-                if (done >= kLaneTrial && listed > done * 20 && A.hint == nullptr)
-                    at = atomicAdd(&A.counters[8], (int)min((int64_t)32, A.end - gb));
-            }
-            at = __shfl_sync(kFull, at, 0);
-            if (at >= 0)
-            {
-                if (act)
-                {
-                    const int i = (int)gb + lane, u = A.oid[i];
-                    A.deg[u] = 0;
-                    A.status[u] = kPlaneOverflow; // placeholder until the pass over the list
-                    list[at + lane] = i;
-                }
-                continue;
-            }
-        }
-        C.init((int)(act ? gb + lane : A.end - 1));
+        // Groups lie at multiples of 32 of the curve order and are built whole, so that a cell does not depend on
+        // the range or chunk that asks for it (what its warp searches for depends on the other cells of the
+        // group); cells outside the range are not written.
+        const bool mine = gb + lane >= A.begin && gb + lane < A.end;
+        bool act = gb + lane < A.n;
+        C.init((int)(act ? gb + lane : A.n - 1));
         float hint = INFINITY; // search radius
         if (A.hint != nullptr)
         {
@@ -429,21 +411,74 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
             C.n_hit += C.rsafe <= hint ? 1u : 0u;
             C.n_miss += C.rsafe <= hint ? 0u : 1u;
         }
-        if (EXPORT && act)
+        if (EXPORT && act && mine)
             C.export_cell();
         __syncwarp();
-        if (act)
-            C.output(list, &A.counters[8]);
+        if (act && mine)
+            C.output(list, &A.counters[kCountListed]);
         __syncwarp();
-        if (lane == 0)
-            atomicAdd(&A.counters[9], 1);
     }
     C.flush();
 }
 
+// Survey of a build's points: per sampled group of 32 consecutive points of the curve (a warp's cells), whether
+// they lie flat, and the level of the octree cell around them (the highest bit in which the first and last key
+// differ). Flat: with the eigenvalues a >= b >= c of their covariance, c (1/a + 1/b) < 0.1. Integer sums: the
+// outcome does not depend on the order of the warps.
+__global__ void __launch_bounds__(256) k_lane_survey(const float4 *__restrict__ pts,
+                                                     const unsigned long long *__restrict__ keys, int64_t n, int groups,
+                                                     int *__restrict__ counters)
+{
+    const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
+    int flat = 0, level = 0, level2 = 0;
+    for (int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < groups; t += warps)
+    {
+        const int64_t i = (n / 32) * t / groups * 32;
+        const float4 p = pts[i + lane];
+        auto sum = [](float v) -> float {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                v += __shfl_xor_sync(kFull, v, o);
+            return v;
+        };
+        float x = p.x - sum(p.x) * (1.0f / 32.0f), y = p.y - sum(p.y) * (1.0f / 32.0f),
+              z = p.z - sum(p.z) * (1.0f / 32.0f);
+        const float big = __uint_as_float(
+            __reduce_max_sync(kFull, __float_as_uint(fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z))))));
+        const float sc = big > 0.0f ? 1.0f / big : 0.0f;
+        x *= sc;
+        y *= sc;
+        z *= sc;
+        const float xx = sum(x * x), yy = sum(y * y), zz = sum(z * z), xy = sum(x * y), xz = sum(x * z),
+                    yz = sum(y * z);
+        // det = abc, minors = ab + bc + ca, trace = a + b + c
+        const float m0 = yy * zz - yz * yz, m1 = xx * zz - xz * xz, m2 = xx * yy - xy * xy;
+        const float det = xx * m0 - xy * (xy * zz - yz * xz) + xz * (xy * yz - yy * xz), minors = m0 + m1 + m2;
+        flat += det * (xx + yy + zz) < 0.1f * minors * minors ? 1 : 0;
+        const unsigned long long d = keys[i] ^ keys[i + 31];
+        const int l = d != 0ull ? 63 - __clzll(d) : 0;
+        level += l;
+        level2 += l * l;
+    }
+    if (lane == 0)
+    {
+        atomicAdd(&counters[kCountFlat], flat);
+        atomicAdd(&counters[kCountLevel], level);
+        atomicAdd(&counters[kCountLevelSq], level2);
+    }
+}
+
+int lane_survey_launch(const Workspace &ws, int64_t n, cudaStream_t st)
+{
+    const int groups = (int)std::min<int64_t>(n / 32, kSurveyGroups);
+    ++g_launches;
+    k_lane_survey<<<kSurveyGroups / 8, 256, 0, st>>>(ws.pts, ws.keys0, n, groups, ws.counters);
+    return groups;
+}
+
 void lane_launch(const CellArgs &A, int *list, int num_sms, cudaStream_t st)
 {
-    const int64_t need = (A.end - A.begin + 31) / 32;
+    const int64_t need = (A.end - (A.begin & ~(int64_t)31) + 31) / 32;
     const int64_t grid = std::min<int64_t>((int64_t)num_sms * kLaneBlocks, need);
     const bool exports = A.geometry_out || A.vertices_out || A.vertex_planes_out || A.vertex_count_out;
     void (*kern)(CellArgs, int *) = A.guesses ? (exports ? k_cells_lane<true, true> : k_cells_lane<true, false>)

@@ -28,7 +28,7 @@ _last_stats: dict = {}
 _last_diag: dict = {}
 #: Names of the values returned by ``last_profile()`` (pg_last_profile in include/paragram_b200.h).
 PROFILE_NAMES = ["launches", "lbvh_ms", "cells_ms", "deferred_ms", "csr_ms", "deferred_cells", "chunks",
-                 "deferred_256", "deferred_512", "routed_cells"]
+                 "deferred_256", "deferred_512", "routed_cells", "lane_cells", "listed_cells"]
 
 
 def _check(ok: bool, msg: str):

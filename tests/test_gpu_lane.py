@@ -1,6 +1,9 @@
 """The cell-per-lane first pass (builds of at least kLaneMinCells cells, pg_lane.cu) against the oracle, at
 the sizes and inputs where its rules end: the last warp's idle lanes, coincident
-points, cells of more than 42 vertices, reaches that hold too many points, chunks."""
+points, cells of more than 42 vertices, reaches that hold too many points, chunks,
+ranges, and the survey that declines it (surfaces; few cells of varying density)."""
+
+import ctypes
 
 import numpy as np
 import pytest
@@ -41,6 +44,8 @@ def _cloud(kind, n, seed=5):
         p = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3).copy()
     elif kind == "surface":
         p = W.surface_cloud(n, np.random.Generator(np.random.PCG64(seed)))
+    elif kind == "clustered":
+        p = W.clustered(n, seed)
     elif kind == "dense_spots":  # a tenth of the points in 40 spots a thousandth of the spacing wide
         p = W.uniform(n, seed)
         k = n // 10
@@ -70,11 +75,77 @@ def _gpu(p, w, dev, **kw):
 @pytest.mark.parametrize("kind,n", [("uniform", MIN - 1), ("uniform", MIN), ("uniform", MIN + 1), ("power", MIN + 31),
                                     ("heavy", 40_000), ("lattice", 35_937), ("exact_lattice", 35_937),
                                     ("surface", 36_001), ("dense_spots", 40_000), ("coincident", 36_000),
-                                    ("wheel", 36_600)])
+                                    ("wheel", 36_600), ("clustered", MIN + 5), ("clustered", 60_001)])
 def test_lane_pass_equals_oracle(dev, oracle, kind, n):
     p, w = _cloud(kind, n)
     got, _ = _gpu(p, w, dev)
     assert diff_cells(got, oracle.diagram(p, w)).size == 0
+
+
+@pytest.mark.parametrize("kind,n,taken", [("uniform", MIN - 1, False), ("uniform", MIN, True), ("heavy", 40_000, True),
+                                          ("lattice", 35_937, True), ("clustered", MIN + 5, False),
+                                          ("clustered", 60_001, True), ("surface", 36_001, False),
+                                          ("surface", 100_000, False), ("surface", 400_000, True)])
+def test_lane_pass_choice(dev, kind, n, taken):
+    """Which builds the pass takes, that most of their cells stay in it, and the same diagram either way
+    (blocks_per_sm = 3 keeps a build from the pass)."""
+    import paragram_b200.cuda as pc
+
+    p, w = _cloud(kind, n)
+    got, _ = _gpu(p, w, dev)
+    prof = pc.last_profile()
+    assert prof["lane_cells"] == (n if taken else 0)
+    assert prof["listed_cells"] < 0.6 * n if taken else prof["listed_cells"] == 0
+    ref, _ = _gpu(p, w, dev, blocks_per_sm=3)
+    assert pc.last_profile()["lane_cells"] == 0
+    assert all(np.array_equal(x, y) for x, y in zip(got, ref))
+
+
+@pytest.mark.parametrize("kind,n", [("clustered", 70_001), ("surface", 100_000), ("surface", 300_000)])
+def test_exports_do_not_depend_on_timing_chunks_or_ranges(dev, kind, n):
+    """Volumes, centroids and vertices bit by bit: of a second call, of a build in chunks, and of a build of a
+    range of the curve (whose ends lie inside groups of 32 cells)."""
+    import paragram_b200.cuda as pc
+    from paragram_b200 import _lib
+
+    p, _ = _cloud(kind, n)
+    t = torch.from_numpy(p).to(dev)
+    names = ("centroids", "volumes", "vertices", "vertex_bound", "vertex_planes", "vertex_count")
+    bits = lambda x: x.contiguous().view(torch.int32)  # noqa: E731
+    _, a = pc.build_with_stats(t, geometry=True, vertices=24, features=True)
+    for kw in ({}, {}, dict(num_chunks=5)):
+        _, b = pc.build_with_stats(t, geometry=True, vertices=24, **kw)
+        assert all(torch.equal(bits(a[k]), bits(b[k])) for k in names), kw
+    begin, end = 1003, 1003 + max(MIN, int(0.9 * n))
+    lib = _lib.load()
+    size = ctypes.c_size_t(0)
+    assert lib.pg_workspace_size(n, ctypes.byref(size)) == 0
+    ws = torch.empty(size.value, dtype=torch.uint8, device=dev)
+    status = torch.empty(n, dtype=torch.int32, device=dev)
+    geom = torch.full((n, 4), -1.0, dtype=torch.float32, device=dev)
+    opt = _lib.PgOptions(8, -1, 0, 0, 0)
+    opt.geometry_out = geom.data_ptr()
+    assert lib.pg_build_range(n, t.data_ptr(), None, ctypes.byref(opt), ws.data_ptr(), size.value, begin, end,
+                              status.data_ptr(), torch.cuda.current_stream(dev).cuda_stream) == 0
+    inside = torch.zeros(n, dtype=torch.bool, device=dev)
+    inside[a["order"][begin:end].long()] = True
+    assert torch.equal(bits(geom[inside, :3]), bits(a["centroids"][inside]))
+    assert torch.equal(bits(geom[inside, 3]), bits(a["volumes"][inside]))
+    assert bool((geom[~inside] == -1.0).all())
+
+
+def test_declined_build_keeps_its_guesses(dev):
+    """Cells left to the warp-per-cell pass are clipped by the caller's guesses there too: the true neighbours
+    as guesses save it nodes (the counters of a build that the lane pass takes hold its shared searches too)."""
+    import paragram_b200.cuda as pc
+
+    p, _ = _cloud("surface", 40_000)
+    (adj, off, st), cold = _gpu(p, None, dev)
+    g = dict(initial_guesses=torch.from_numpy(adj).to(dev), initial_guesses_offsets=torch.from_numpy(off).to(dev))
+    got, warm = _gpu(p, None, dev, **g)
+    assert pc.last_profile()["lane_cells"] == 0
+    assert all(np.array_equal(x, y) for x, y in zip(got, (adj, off, st)))
+    assert warm["nodes"] < 0.9 * cold["nodes"]
 
 
 def test_lane_pass_equals_warp_pass_and_chunks(dev):
