@@ -76,16 +76,17 @@ constexpr uint32_t kBigFlag = 0x40000000u; // deg[] flag: row lives in the defer
 // the pass over the list takes as long as the slowest of them. Variance of the levels 2 to 3 in uniform points
 // (warp-per-cell pass 2.28 ms, cell-per-lane 2.11 at 40,000), 4.2 in 64 Gaussians of similar widths (2.18, 2.20),
 // 4.9 in 500 narrow ones (2.47, 3.03), 14 to 21 with widths from 0.005 to 0.1 (2.50, 2.80 at 40,000; 3.09, 3.14 at
-// 56,000; 3.24, 3.27 at 60,000; 4.02, 3.70 at 80,000).
+// 56,000; 3.24, 3.27 at 60,000; 4.02, 3.70 at 80,000; with the previous step's diagram as guesses 2.36, 2.39 at
+// 36,000; 2.91, 2.87 at 48,000; 3.24, 3.03 at 56,000).
 constexpr int kSurveyGroups = 512;
 constexpr int kLaneFlatShare = 10;         // declined above one flat group in ten
 constexpr int kLaneLevelVar2 = 9;          // declined below kLaneAnyCells above half this variance of the levels
-constexpr int64_t kLaneAnyCells = 60000;
+constexpr int64_t kLaneAnyCells = 60000, kLaneAnyCellsGuess = 46000; // (the latter with initial guesses)
 struct LaneChoice
 {
     const int *counters; // the workspace's
     int groups;          // groups sampled
-    int few;             // the build has fewer than kLaneAnyCells cells
+    int few;             // the build has fewer than kLaneAnyCells(Guess) cells
 
     __host__ __device__ bool declined() const
     {
