@@ -40,20 +40,11 @@ constexpr int kMaxWarpsPerSM = 32;  // upper bound of resident cell warps per SM
 constexpr int kBigWarps = 4;        // warps per block of the 256-slot tier (state in shared memory)
 constexpr int kMidWarps = 4;        // warps per block of the 128-slot tier (13 KB of shared memory each)
 constexpr int kMidBlocksPerSM = 3;  // its resident blocks per SM (up to 170 registers per thread)
-#ifndef PG_LANE_V
-#define PG_LANE_V 42
-#endif
-#ifndef PG_LANE_WARM
-#define PG_LANE_WARM 16
-#endif
-#ifndef PG_LANE_MIN
-#define PG_LANE_MIN 32768
-#endif
 // Vertex slots of a cell of the cell-per-lane pass: with 42 eight one-warp blocks fit in an SM's shared memory,
 // with 48 seven (2M clustered cells 38.6 against 41.0 ms), with 36 nine, but too many cells outgrow them (44.6).
-constexpr int kLaneV = PG_LANE_V;
-constexpr int kLaneWarm = PG_LANE_WARM; // nearest points that clip it first
-constexpr int64_t kLaneMinCells = PG_LANE_MIN; // smallest build of that pass
+constexpr int kLaneV = 42;
+constexpr int kLaneWarm = 16; // nearest points that clip it first
+constexpr int64_t kLaneMinCells = 32768; // smallest build of that pass
 // entries of the workspace's counters that the cell-per-lane pass uses: the cells it listed and, over the groups
 // that the survey sampled, the flat ones, the sum of their levels and of the levels' squares
 constexpr int kCountListed = 8, kCountFlat = 9, kCountLevel = 10, kCountLevelSq = 11;

@@ -36,24 +36,12 @@
 namespace pg
 {
 
-#ifndef PG_LANE_BLOCKS
-#define PG_LANE_BLOCKS 8
-#endif
-#ifndef PG_LANE_SHELL
-#define PG_LANE_SHELL 2.5f
-#endif
-#ifndef PG_LANE_FAR
-#define PG_LANE_FAR 6.0f
-#endif
-#ifndef PG_LANE_MARKS
-#define PG_LANE_MARKS 96
-#endif
-constexpr int kLaneBlocks = PG_LANE_BLOCKS; // resident one-warp blocks per SM (28 KB of shared memory each)
+constexpr int kLaneBlocks = 8; // resident one-warp blocks per SM (28 KB of shared memory each)
 // Squared radius of the first search over the last near point's. 500,000 clustered cells: 2.0 14.5, 2.5 13.8,
 // 3.0 14.8 ms (a smaller one leaves more cells to the second search, a larger one more points to test).
-constexpr float kLaneShell = PG_LANE_SHELL;
-constexpr float kLaneFar = PG_LANE_FAR;     // the largest that a cell may need after it (beyond: listed)
-constexpr int kLaneMarks = PG_LANE_MARKS;   // points of a search within a cell's reach
+constexpr float kLaneShell = 2.5f;
+constexpr float kLaneFar = 6.0f; // the largest that a cell may need after it (beyond: listed)
+constexpr int kLaneMarks = 96;   // points of a search within a cell's reach
 
 // Optional per-phase SM cycle counters, as in pg_cells.cu (compile with -DPG_PHASE_CYCLES): the clips by the
 // nearest points, the search, its tests, the clips by its points, and whole cells, per cell.
@@ -90,6 +78,7 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
     if (A.choice.declined())
         return; // every cell is left to k_cells_list
     LaneCell C(m, A, lane);
+    const int root = A.cloud_root[0];
     unsigned cmask[kLaneLeaves / 2];
     int cand[kLaneCut];
     for (;;)
@@ -133,7 +122,6 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
             {
                 const int o = A.guesses[k];
                 const int j = o >= 0 && o < A.n ? A.rank[o] : -1;
-                // (a guess in another cloud is a point all the same)
                 if (j >= 0 && j != C.i)
                 {
                     cand[nk++] = j;
@@ -208,23 +196,13 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
                 nk = 0;
                 int sp = 0, marks = 0;
                 bool over = false;
-                float rr = -1.0f;
-                for (unsigned todo = __ballot_sync(kFull, search);;)
+                float rr = search ? hi : -1.0f;
+                if (lane == 0)
+                    m.stk[0] = root;
+                sp = 1;
+                __syncwarp();
+                while (sp > 0)
                 {
-                    if (sp == 0)
-                    {
-                        if (todo == 0u || over)
-                            break;
-                        // (a warp's cells may belong to several clouds)
-                        const int root = __shfl_sync(kFull, C.root, __ffs(todo) - 1);
-                        const bool mine = search && C.root == root;
-                        todo &= ~__ballot_sync(kFull, mine);
-                        rr = mine ? hi : -1.0f;
-                        if (lane == 0)
-                            m.stk[0] = root;
-                        sp = 1;
-                        __syncwarp();
-                    }
                     int nl = 0;
                     while (sp > 0 && nl <= kLaneLeaves - 4)
                     {
@@ -242,7 +220,6 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
                         if (sp + 4 > kLaneStack)
                         {
                             over = true;
-                            sp = 0;
                             break;
                         }
                         const float f4[4] = {a3.x, a3.y, b3.x, b3.y};

@@ -91,9 +91,9 @@ struct LaneCell
     LaneMem &m;
     const CellArgs &A;
     const int lane;
-    int i = -1, soid = 0, root = 0;
+    int i = -1, soid = 0;
     float4 s;
-    const float *box;
+    const float *const box;
     bool alive = false, defer = false, empty = false;
     int nv = 0;              // vertices (slots 0 .. nv - 1)
     unsigned live = 0;       // plane slots that a vertex uses
@@ -105,10 +105,9 @@ struct LaneCell
     long long cyc[kLaneCycNum] = {};
 #endif
 
-    __device__ __forceinline__ LaneCell(LaneMem &mem, const CellArgs &args, int l) : m(mem), A(args), lane(l)
+    __device__ __forceinline__ LaneCell(LaneMem &mem, const CellArgs &args, int l) : m(mem), A(args), lane(l), box(args.box)
     {
         s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        box = A.box;
         clear_dx();
     }
     __device__ __forceinline__ void clear_dx()
@@ -149,18 +148,15 @@ struct LaneCell
         return (1u << (tr & 31u)) | (1u << ((tr >> 5) & 31u)) | (1u << (tr >> 10));
     }
 
-    // Cell of sorted slot c: the box (planes 0..5, corners 0..7).
+    // Cell of sorted slot c of a build of one cloud: the box (planes 0..5, corners 0..7).
     __device__ __forceinline__ void init(int c)
     {
         i = c;
         s = A.pts[i];
         soid = A.oid[i];
-        const int cloud = cloud_of(A.cloud_off, A.num_clouds, i);
-        box = A.box + 8 * cloud;
-        root = A.cloud_root[cloud];
         empty = false;
-        defer = ref_is_leaf(root); // a cloud of one leaf has no records: the warp-per-cell pass
-        alive = !defer;
+        defer = false;
+        alive = true;
         rsafe = INFINITY;
         nv = 8;
         live = 0x3Fu;
