@@ -20,7 +20,7 @@
 // Eight lanes per cell: 26 ms (instruction-cache misses between the steps).
 //
 // Builds whose points would mostly be listed are declined as a whole (LaneChoice, pg_common.cuh). A cell that
-// does not fit (more than kLaneV vertices or kLaneP planes at a time, a
+// does not fit (more than kLaneV vertices, a
 // reach that holds more than kLaneMarks points: cells at the hull, beside a far denser
 // region, or long cells of surface data) is listed for the warp-per-cell pass.
 //
@@ -197,10 +197,10 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
                 int sp = 0, marks = 0;
                 bool over = false;
                 float rr = search ? hi : -1.0f;
-                if (lane == 0)
-                    m.stk[0] = root;
+                // pending nodes: entry k in lane k % 32's stk0 (k < 32) or stk1
+                int stk0 = root, stk1 = 0;
+                auto pending = [&](int k) -> int { return __shfl_sync(kFull, k < 32 ? stk0 : stk1, k & 31); };
                 sp = 1;
-                __syncwarp();
                 while (sp > 0)
                 {
                     int nl = 0;
@@ -208,7 +208,8 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
                     {
                         // two nodes at a time: their loads overlap
                         const int two = sp > 1 ? 1 : 0;
-                        const float4 *pa = A.rec + 4 * (size_t)m.stk[sp - 1], *pb = A.rec + 4 * (size_t)m.stk[sp - 1 - two];
+                        const float4 *pa = A.rec + 4 * (size_t)pending(sp - 1),
+                                     *pb = A.rec + 4 * (size_t)pending(sp - 1 - two);
                         const float4 a0 = pa[0], a1 = pa[1], a2 = pa[2], a3 = pa[3];
                         const float4 b0 = pb[0], b1 = pb[1], b2 = pb[2], b3 = pb[3];
                         sp -= 1 + two;
@@ -230,10 +231,18 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
                                 const int f = __float_as_int(f4[c]);
                                 C.n_nodes += mine[c] ? 1u : 0u;
                                 C.n_leaves += mine[c] && f < 0 ? 1u : 0u;
-                                if (lane == 0)
-                                    (f < 0 ? m.lv[nl] : m.stk[sp]) = f;
-                                nl += f < 0 ? 1 : 0;
-                                sp += f < 0 ? 0 : 1;
+                                if (f < 0)
+                                {
+                                    if (lane == 0)
+                                        m.lv[nl] = f;
+                                    ++nl;
+                                }
+                                else
+                                {
+                                    if (lane == (sp & 31))
+                                        (sp < 32 ? stk0 : stk1) = f;
+                                    ++sp;
+                                }
                             }
                         __syncwarp();
                     }
@@ -331,10 +340,10 @@ __global__ void __launch_bounds__(32, kLaneBlocks) k_cells_lane(CellArgs A, int 
                     }
                     PG_LANE_T1(C, kLaneCycTests, t0);
                 }
+                __syncwarp();
+                C.clear_dx(); // (the search's list lies there)
                 if ((over && search) || nk > kLaneCut)
-                {
                     C.give_up();
-                }
                 if (!C.alive)
                     nk = 0;
                 lo = __uint_as_float(__float_as_uint(hi) + 1u); // the next shell begins beyond hi

@@ -1,9 +1,9 @@
 // pg_lane.cuh -- one lane's cell: the polytope of the cell-per-lane pass (pg_lane.cu).
 //
-// Shared memory is laid out [slot][lane], so that the lanes' accesses never share a bank
-// whatever slots they are at. A vertex takes 16 bytes, its plane triple in the low bits
-// of its error radius; planes are not stored but recomputed from their points, whose
-// loads L1 and L2 serve, so that 256 cells fit in an SM's shared memory.
+// Shared memory is laid out [slot][lane], so that the lanes' accesses to a slot's vertex
+// never share a bank. Planes are not stored but recomputed from their points, whose loads
+// L1 and L2 serve, and what a search and a clip need only in turn lies in one place, so
+// that 256 cells fit in an SM's shared memory.
 #pragma once
 
 #include "pg_clip.cuh"
@@ -11,30 +11,31 @@
 namespace pg
 {
 
-constexpr int kLaneP = 32;       // plane slots of a cell (one bit each in a live mask)
-constexpr int kLaneStack = 64;   // pending BVH nodes of a warp's search
-constexpr int kLaneLeaves = 128; // leaves that a warp's search lists before they are scanned
-constexpr int kLaneCut = 48;     // points of a search that may cut a cell
+constexpr int kLaneP = 24;      // plane slots of a cell: V vertices lie on V / 2 + 2 planes, and one more in a clip
+constexpr int kLaneStack = 64;  // pending BVH nodes of a warp's search
+constexpr int kLaneLeaves = 92; // leaves that a warp's search lists before they are scanned
+constexpr int kLaneCut = 48;    // points of a search that may cut a cell
+static_assert(kLaneP >= kLaneV / 2 + 3 && kLaneP <= 32, "a live mask has a bit for each plane");
 
 // One warp's 32 cells (lane = column) and its search of the BVH.
 struct LaneMem
 {
-    float4 vx[kLaneV][32];       // vertex relative to the seed; w: error radius psi, its low 15 bits the plane triple
-    int pid[kLaneP][32];         // >= 0: sorted point index; < 0: -1 - box code
-    unsigned dx[kLaneP / 4][32]; // per plane slot (bytes): xor of its boundary successor and predecessor
-    float4 pt[32];               // points of the leaf pair in work
-    int lv[kLaneLeaves + 4];     // leaves within reach
-    int stk[kLaneStack];
+    float4 vx[kLaneV][32];          // vertex relative to the seed; w: error radius psi
+    unsigned short vt[kLaneV][32];  // its plane slots, five bits each
+    int pid[kLaneP][32];            // >= 0: sorted point index; < 0: -1 - box code
+    union
+    {
+        unsigned dx[kLaneP / 4][32]; // in a clip (else zero), per plane slot (bytes): xor of its boundary successor and predecessor
+        struct
+        {
+            float4 pt[32];           // points of the leaf pair in work
+            int lv[kLaneLeaves + 4]; // leaves within reach
+        };
+    };
 };
+static_assert(sizeof(LaneMem) + 1024 <= 228 * 1024 / 8, "eight blocks of one warp per SM");
 
 __device__ __forceinline__ unsigned tri5(unsigned a, unsigned b, unsigned c) { return a | (b << 5) | (c << 10); }
-
-// psi rounded up to a float whose low 15 bits hold the triple: read as a float, the word itself
-// is an upper bound of psi (at most 2^-7 above it).
-__device__ __forceinline__ float pack_psi(float psi, unsigned tri)
-{
-    return __uint_as_float((__float_as_uint(fminf(psi, 1e30f)) & ~0x7FFFu) + 0x8000u + tri);
-}
 
 struct LPlane
 {
@@ -117,7 +118,7 @@ struct LaneCell
             m.dx[k][lane] = 0u;
     }
     __device__ __forceinline__ float4 &vxl(int v) { return m.vx[v][lane]; }
-    __device__ __forceinline__ unsigned tri_of(int v) { return __float_as_uint(m.vx[v][lane].w) & 0x7FFFu; }
+    __device__ __forceinline__ unsigned tri_of(int v) { return m.vt[v][lane]; }
     __device__ __forceinline__ int &pidl(unsigned p) { return m.pid[p][lane]; }
     __device__ __forceinline__ unsigned char &dxa(unsigned x)
     {
@@ -182,7 +183,8 @@ struct LaneCell
             float x2 = X * X + Y * Y + Z * Z;
             float xn = x2 > 0.0f ? x2 * rsqrtf(x2) * (1.0f + 4e-6f) : 0.0f;
             float psi = (2.0f * ex + 4.0f * kEps * xn) * (1.0f + 1e-6f);
-            vxl(c8) = make_float4(X, Y, Z, pack_psi(psi, tri5(p0, p1, p2)));
+            vxl(c8) = make_float4(X, Y, Z, psi);
+            m.vt[c8][lane] = tri5(p0, p1, p2);
         }
     }
 
@@ -278,13 +280,13 @@ struct LaneCell
             alive = false;
             return;
         }
-        if (live == 0xFFFFFFFFu)
+        const unsigned P = __ffs(~live) - 1;
+        if (P >= (unsigned)kLaneP)
         {
-            give_up();
+            give_up(); // (not reached: see kLaneP)
             return;
         }
         ++n_clips;
-        const unsigned P = __ffs(~live) - 1;
         pidl(P) = j;
         // Boundary of the removed region. Every removed triangle xors, for each of its planes, the other
         // two into that plane's byte: inside the region each neighbour enters twice, so a plane on the
@@ -380,9 +382,10 @@ struct LaneCell
             {
                 (slot < 32 ? ill0 : ill1) |= 1u << (slot & 31);
                 if (!(X.w < 1e30f))
-                    X = make_float4(0.0f, 0.0f, 0.0f, 1e30f);
+                    X = make_float4(0.0f, 0.0f, 0.0f, INFINITY); // (not NaN: such a vertex may be cut by any point)
             }
-            vxl(slot) = make_float4(X.x, X.y, X.z, pack_psi(X.w, tri5(P, x, y)));
+            vxl(slot) = X;
+            m.vt[slot][lane] = tri5(P, x, y);
             x = y;
             y = w;
             px = py;
@@ -394,12 +397,12 @@ struct LaneCell
         {
             const int v = take(ill0, ill1);
             const float4 X = vxl(v);
-            const unsigned tr = __float_as_uint(X.w) & 0x7FFFu;
+            const unsigned tr = tri_of(v);
             float vr;
             const float4 Y = make_vertex64(pidl(tr & 31u), pidl((tr >> 5) & 31u), pidl(tr >> 10), A.pts, A.oid, box, s,
                                            X, 0.0f, vr);
             if (Y.w < X.w)
-                vxl(v) = make_float4(Y.x, Y.y, Y.z, pack_psi(Y.w, tr));
+                vxl(v) = Y;
             ++n_v64;
         }
         // holes left by removed vertices are filled from the end
@@ -409,7 +412,10 @@ struct LaneCell
             (r1 ? r1 : r0) &= ~(1u << (hole & 31));
             --nv;
             if (hole != nv)
+            {
                 vxl(hole) = vxl(nv);
+                m.vt[hole][lane] = m.vt[nv][lane];
+            }
         }
     }
 
@@ -448,7 +454,7 @@ struct LaneCell
             float4 X = vxl(v);
             if (!(X.w <= 32.0f * kEps * (fabsf(X.x) + fabsf(X.y) + fabsf(X.z))))
             {
-                const unsigned tr = __float_as_uint(X.w) & 0x7FFFu;
+                const unsigned tr = tri_of(v);
                 X = vertex64_plain(pidl(tr & 31u), pidl((tr >> 5) & 31u), pidl(tr >> 10), A.pts, A.oid, box, s, X);
                 vxl(v) = X;
             }
@@ -462,7 +468,7 @@ struct LaneCell
                     A.vertices_out[at] = X;
                 if (A.vertex_planes_out != nullptr)
                 {
-                    const unsigned tr = __float_as_uint(X.w) & 0x7FFFu;
+                    const unsigned tr = tri_of(v);
 #pragma unroll
                     for (int e = 0; e < 3; ++e)
                     {

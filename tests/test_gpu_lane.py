@@ -193,6 +193,28 @@ def test_lane_pass_exports(dev, kind):
     assert bool(((xa - xb).norm(dim=2)[on] <= (ba + bb)[on].double() * (1 + 1e-6)).all())
 
 
+def test_lane_pass_keeps_all_bits_of_the_bounds(dev):
+    """The vertex bounds of both passes come from the same formula over the same three planes (in another order:
+    roundings either way): their ratio's median is 1. A bound rounded up to 8 or 9 bits would raise it by a
+    third of 2^-8 to 2^-7; the line is drawn at 2^-10."""
+    p, _ = _cloud("uniform", 40_000)
+    _, a = _gpu(p, None, dev, vertices=42, blocks_per_sm=3)
+    _, b = _gpu(p, None, dev, vertices=42)
+    n, k = len(p), 42
+    bounds = []
+    for r in (a, b):
+        count = r["vertex_count"]
+        used = (torch.arange(k, device=dev)[None] < count[:, None]) & (count[:, None] <= k)
+        q = r["vertex_planes"].long().sort(2).values
+        key = ((q[..., 0] + 8) * (n + 16) + q[..., 1] + 8) * (n + 16) + q[..., 2] + 8
+        key, at = torch.where(used, key, torch.iinfo(torch.int64).max).sort(1)
+        bounds.append((key, torch.gather(r["vertex_bound"], 1, at).double(), used.sum()))
+    (ka, ba, na), (kb, bb, nb) = bounds
+    assert torch.equal(ka, kb) and int(na) == int(nb) > 20 * n
+    ratio = (bb / ba)[ka < torch.iinfo(torch.int64).max]
+    assert abs(float(ratio.median()) - 1.0) < 2.0 ** -10
+
+
 def test_lane_pass_guesses_and_radius(dev):
     """Initial guesses (true neighbours, with repeats, the point itself and ids out of range; too many; none)
     and search radii (exact, far too small, none) leave the diagram as it is."""
