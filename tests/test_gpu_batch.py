@@ -129,3 +129,13 @@ def test_batch_geometry_partition(dev):
         assert abs(part[:, 3].sum() - vol) <= 1e-5 * vol
         cen = (part[:, :3] * part[:, 3:4]).sum(0) / part[:, 3].sum()
         assert np.abs(cen - 0.5 * (lo + hi)).max() <= 1e-5 * np.abs(hi - lo).max()
+
+
+def test_batch_of_volumes_equals_single_calls(dev):
+    """Clouds that a single call builds by the cell-per-lane pass, and smaller ones."""
+    import paragram_b200 as pg
+    from paragram_b200 import workloads as W
+
+    tens = [torch.from_numpy(c).to(dev) for c in (W.uniform(40_000, 1), W.uniform(500, 2), W.clustered(70_000, 3))]
+    for d, p in zip(pg.build_batch(tens), tens):
+        assert all(np.array_equal(a, b) for a, b in zip(_np(d), _np(pg.voronoi_diagram(p))))

@@ -159,3 +159,64 @@ def test_bounds_keep_non_finite_values(dev, n):
     hi = np.float32(pts[finite[:, 2], 2].max()) + np.float32(1) + np.float32(1e-5)
     assert np.array_equal(box[:3], np.array(lo, np.float32)) and box[5] == hi
     assert np.isnan(box[3]) and np.isinf(box[4]) and np.isnan(box[6])
+
+
+def _morton_keys(pts):
+    """The build's keys (21 bits per axis, x the highest) of float32 points, in the same float32 operations."""
+    lo, ext = pts.min(0), np.float32((pts.max(0) - pts.min(0)).max())
+    scale = np.float32(2 ** 21 - 1) / ext
+    q = np.clip((pts - lo) * scale, np.float32(0), np.float32(2 ** 21 - 1)).astype(np.uint64)
+    key = np.zeros(len(pts), np.uint64)
+    for b in range(21):
+        for k in range(3):
+            key |= ((q[:, k] >> np.uint64(b)) & np.uint64(1)) << np.uint64(3 * b + 2 - k)
+    return key
+
+
+@pytest.mark.parametrize("n", [2, 33, 4095, 4096, 4097, 8192, 599_999, 600_000])
+def test_order_is_the_stable_sort_by_key(dev, n):
+    """Points on a coarse grid (many equal keys) at the sizes where the sort changes: one block up to 4,096
+    keys, small tiles below 600,000. Equal keys keep the points' order."""
+    from paragram_b200 import _lib
+
+    lib = _lib.load()
+    rng = np.random.default_rng(n)
+    pts = (rng.integers(0, 24, (n, 3)) / 16.0).astype(np.float32)
+    pts[0], pts[-1] = 0.0, 1.5
+    p = torch.from_numpy(pts).to(dev)
+    size = ctypes.c_size_t(0)
+    assert lib.pg_workspace_size(n, ctypes.byref(size)) == 0
+    ws = torch.empty(size.value, dtype=torch.uint8, device=dev)
+    status = torch.empty(n, dtype=torch.int32, device=dev)
+    order = torch.empty(n, dtype=torch.int32, device=dev)
+    opt = _lib.PgOptions(8, -1, 0, 0, 0)
+    opt.order_out = order.data_ptr()
+    # (a range build without cells: the tree alone)
+    assert lib.pg_build_range(n, p.data_ptr(), None, ctypes.byref(opt), ws.data_ptr(), size.value, 0, 0,
+                              status.data_ptr(), torch.cuda.current_stream(dev).cuda_stream) == 0
+    assert np.array_equal(order.cpu().numpy(), np.argsort(_morton_keys(pts), kind="stable"))
+
+
+def test_one_workspace_for_smaller_builds(dev):
+    """A workspace sized for 600,050 points serves smaller builds on both sides of the sort's rules."""
+    import paragram_b200 as pg
+    from paragram_b200 import _lib
+    from paragram_b200 import workloads as W
+
+    lib = _lib.load()
+    stream = torch.cuda.current_stream(dev).cuda_stream
+    size = ctypes.c_size_t(0)
+    assert lib.pg_workspace_size(600_050, ctypes.byref(size)) == 0
+    ws = torch.empty(size.value, dtype=torch.uint8, device=dev)
+    cloud = torch.from_numpy(W.uniform(600_050, 3)).to(dev)
+    for n in (600_050, 600_000, 599_999, 4097, 4096):
+        p = cloud[:n].contiguous()
+        offsets = torch.empty(n + 1, dtype=torch.int32, device=dev)
+        status = torch.empty(n, dtype=torch.int32, device=dev)
+        opt, e = _lib.PgOptions(8, -1, 0, 0, 0), ctypes.c_int64(0)
+        assert lib.pg_build(n, p.data_ptr(), None, None, None, ctypes.byref(opt), ws.data_ptr(), size.value,
+                            offsets.data_ptr(), status.data_ptr(), ctypes.byref(e), stream) == 0, _lib.last_error(lib)
+        adj = torch.empty(e.value, dtype=torch.int32, device=dev)
+        assert lib.pg_emit_adjacency(n, ws.data_ptr(), offsets.data_ptr(), adj.data_ptr(), stream) == 0
+        d = pg.voronoi_diagram(p)
+        assert torch.equal(adj, d.adjacency) and torch.equal(offsets, d.offsets) and torch.equal(status, d.status)
