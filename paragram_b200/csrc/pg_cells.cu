@@ -1394,7 +1394,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, MINB) k_cells_fast(CellAr
 
 
 // The cells that the cell-per-lane pass listed, or all of the build's where it was declined, as the first pass
-// builds them.
+// builds them. HINT (builds with a search radius per cell): only the latter, the radius having been too small
+// for most of the former; a launch without HINT takes those.
 // A body of its own: the first pass's code is kept as it is (a branch on the cell's source in its loop made
 // builds with a geometry export 5% slower, from the changed layout of the code alone).
 template <bool GUESS, bool HINT>
@@ -1408,6 +1409,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kMinBlocksLo) k_cells_lis
         m.cnt[lane] = 0;
     clear_edges(m, lane);
     const bool all = A.choice.declined();
+    if (A.hint != nullptr && HINT != all)
+        return;
     const int count = all ? (int)(A.end - A.begin) : A.counters[kCountListed];
     for (;;)
     {
@@ -1657,10 +1660,13 @@ void cells_list_launch(const Workspace &ws, const CellLaunch &cl, int *status, i
     A.big_cap = cl.big_cap;
     A.list = ws.flags;
     cudaMemsetAsync(ws.counters, 0, sizeof(int), st);
-    ++g_launches;
-    void (*kern)(CellArgs) = cl.guesses ? (cl.use_hint ? k_cells_list<true, true> : k_cells_list<true, false>)
-                                        : (cl.use_hint ? k_cells_list<false, true> : k_cells_list<false, false>);
-    kern<<<(unsigned)(num_sms * kMinBlocksLo), kWarpsPerBlock * 32, 0, st>>>(A);
+    for (int hint = 0; hint <= cl.use_hint; ++hint)
+    {
+        void (*kern)(CellArgs) = cl.guesses ? (hint ? k_cells_list<true, true> : k_cells_list<true, false>)
+                                            : (hint ? k_cells_list<false, true> : k_cells_list<false, false>);
+        ++g_launches;
+        kern<<<(unsigned)(num_sms * kMinBlocksLo), kWarpsPerBlock * 32, 0, st>>>(A);
+    }
 }
 
 // The deferred counts stay on the device: fixed grids read them. The middle
