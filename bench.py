@@ -64,6 +64,8 @@ WORKLOADS = {
     "surface_cloud_500k": dict(kind="surface", n=500_000, weighted=False),
     "moving_uniform_1m": dict(kind="moving", n=1_000_000, weighted=False),
 }
+#: what the cell pass's time and work cover in the builds of this file's sizes
+FIRST_PASS = "first pass: k_knn, k_cells_lane, k_cells_list"
 #: workloads built with the learned search radius (plain build timed beside them)
 LEARNED = {"clustered_voronoi_5m", "clustered_voronoi_500k"}
 
@@ -199,10 +201,10 @@ def fp32_peak_tflops(sm_max_mhz: float | None) -> float:
 
 
 def read_traffic_per_launch() -> float | None:
-    """DRAM bytes per cell-pass launch from the committed ncu summary, if present."""
+    """DRAM bytes of the first pass's kernels in one build, from the committed ncu summary, if present."""
     try:
         for line in open(PROFILE_SUMMARY):
-            if line.startswith("dram_bytes_per_launch_full_size:"):
+            if line.startswith("dram_bytes_first_pass:"):
                 return float(line.split(":")[1])
     except OSError:
         pass
@@ -599,6 +601,7 @@ def run_gpu(args, spec, rank, world, local):
     h2d = n * 12 + (n * 4 if h_w is not None else 0)
     # counters of one more (untimed) build: escalations, fallback rate, traversal work; the cell pass alone
     _, cnt = pc.build_with_stats(d_pts, d_w, model=blob)
+    routes = pc.last_profile()
     fp32_only = None
     if args.fp32_only_too:
         # the same build with FP32-only side tests (the reference's arithmetic: no escalation)
@@ -639,6 +642,7 @@ def run_gpu(args, spec, rank, world, local):
                                  "vertex_error": vtx_err},
                   "work_per_cell": {k: round(cnt[k] / n, 3) for k in ("nodes", "leaves", "candidates", "clips",
                                                                        "deferred_cells")},
+                  "cells_by_lane_pass": int(routes["lane_cells"]), "cells_listed_by_it": int(routes["listed_cells"]),
                   "phases_ms": dict(phases, note="one profiled build: LBVH (+ prediction), first cell pass, "
                                                  "deferred-cell pass, CSR count + scan; the CSR fill runs in "
                                                  "the adjacency emission")}
@@ -670,7 +674,7 @@ def run_gpu(args, spec, rank, world, local):
             "step_ms": [round(t, 2) for t in times],
             "config": config,
             "e2e": {"value": e2e_value, "unit": "Mcells/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
-            "roofline": _roofline(flops, nbytes, cell_s, csum, "k_cells_lane (cell pass)",
+            "roofline": _roofline(flops, nbytes, cell_s, csum, FIRST_PASS,
                                   read_traffic_per_launch() if args.workload == "clustered_voronoi_5m" else None),
             "cpu_baseline": _cpu_baseline(args, world, pts, w, n),
             "clocks": csum,
@@ -770,7 +774,7 @@ def run_lattice_gpu(args, spec, rank, world, local, dev):
                        "status_counts": np.bincount(d.status.cpu().numpy(), minlength=6)[:6].tolist(),
                        "phases_ms": {k: round(prof[k], 3) for k in ("lbvh_ms", "cells_ms", "deferred_ms", "csr_ms")}},
             "e2e": {"value": e2e_value, "unit": "Mcells/s", "h2d_bytes_per_step": n * 16, "d2h_bytes_per_step": d2h},
-            "roofline": _roofline(flops, nbytes, cell_s, csum, "k_cells_lane (cell pass)", None),
+            "roofline": _roofline(flops, nbytes, cell_s, csum, FIRST_PASS, None),
             "cpu_baseline": _cpu_baseline(args, world, pts, w, n),
             "clocks": csum,
             "gpu_launches": int(prof["launches"]) * args.steps,
@@ -933,7 +937,7 @@ def run_moving_gpu(args, spec, rank, world, local, dev):
                        "phases_ms": {k_: round(prof[k_], 3) for k_ in ("lbvh_ms", "cells_ms", "deferred_ms",
                                                                        "csr_ms")}},
             "e2e": {"value": e2e_value, "unit": "Mcells/s", "h2d_bytes_per_step": n * 12, "d2h_bytes_per_step": d2h},
-            "roofline": _roofline(flops, nbytes, cell_s, csum, "k_cells_lane (cell pass)", None),
+            "roofline": _roofline(flops, nbytes, cell_s, csum, FIRST_PASS, None),
             "cpu_baseline": _cpu_baseline(args, world, pts, None, n),
             "clocks": csum,
             "gpu_launches": int(prof["launches"]) * args.steps,

@@ -41,7 +41,8 @@ constexpr int kBigWarps = 4;        // warps per block of the 256-slot tier (sta
 constexpr int kMidWarps = 4;        // warps per block of the 128-slot tier (13 KB of shared memory each)
 constexpr int kMidBlocksPerSM = 3;  // its resident blocks per SM (up to 170 registers per thread)
 // Vertex slots of a cell of the cell-per-lane pass: with 42 eight one-warp blocks fit in an SM's shared memory,
-// with 48 seven (2M clustered cells 38.6 against 41.0 ms), with 36 nine, but too many cells outgrow them (44.6).
+// with 48 seven (2M clustered cells 38.6 against 41.0 ms when that was measured), with 36 nine, but too many cells
+// outgrow them (44.6).
 constexpr int kLaneV = 42;
 constexpr int kLaneWarm = 16; // nearest points that clip it first
 constexpr int64_t kLaneMinCells = 32768; // smallest build of that pass

@@ -6,7 +6,7 @@
 // the cells are the same; what differs is who does the work. A warp per cell issues
 // every step of a cell's search once per cell (28,900 warp instructions for a cell of
 // about 27 vertices, 21.8 of 32 lanes active); 32 cells per warp, kept in step, share
-// them: 6,400 per cell.
+// them: 6,300 per cell.
 //
 // What keeps the lanes in step: (1) a cell is first clipped by its kLaneWarm nearest
 // points (k_knn), nearly all of which cut it; (2) the points that can still
@@ -19,14 +19,15 @@
 // 22 ms for 500,000 clustered cells, against 21 ms for a warp per cell and 11 here.
 // Eight lanes per cell: 26 ms (instruction-cache misses between the steps).
 //
-// Builds whose points would mostly be listed are declined as a whole (LaneChoice, pg_common.cuh). A cell that
-// does not fit (more than kLaneV vertices, a
-// reach that holds more than kLaneMarks points: cells at the hull, beside a far denser
-// region, or long cells of surface data) is listed for the warp-per-cell pass.
+// Builds whose points would mostly be listed are declined as a whole (LaneChoice,
+// pg_common.cuh). A cell that does not fit (more than kLaneV vertices, a reach that holds
+// more than kLaneMarks points: cells at the hull, beside a far denser region, or long cells
+// of surface data) is listed for the warp-per-cell pass: 3% of 5M clustered cells, 8% of
+// 500,000, 22% of 60,000.
 //
 // Measured on one B200, first pass with its kNN query and listed cells: 2M clustered
-// points 86 -> 38.6 ms, 500,000 21.0 -> 11.2 ms, 500,000 uniform power 21.8 -> 10.0 ms,
-// jittered 80^3 power lattice 21.4 -> 6.1 ms. Bound by latency: one warp per block, 8
+// points 85.3 -> 37.2 ms, 500,000 21.1 -> 10.8 ms, 500,000 uniform power 21.5 -> 9.6 ms,
+// jittered 80^3 power lattice 19.5 -> 5.8 ms. Bound by latency: one warp per block, 8
 // blocks per SM (28 KB of shared memory each), 38% of the issue slots used.
 #include <algorithm>
 

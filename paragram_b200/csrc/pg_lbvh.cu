@@ -36,7 +36,8 @@ static int sort_blocks(int64_t n) { return (int)((n + sort_tile(n) - 1) / sort_t
 // 586 small tiles, 600,000 only 147 large ones), so that a workspace also serves every smaller build.
 int sort_blocks_upto(int64_t n) { return std::max(sort_blocks(n), sort_blocks(std::min(n, kSortSmall - 1))); }
 
-// Up to kSortOne keys are sorted by one block in shared memory (a launch instead of 8 passes of 3).
+// Up to kSortOne keys are sorted by one block in shared memory (a launch instead of 8 passes of 3): 21 us for
+// 1,000 keys, 70 us for 4,096, where a build is still 30 us faster than one of 4,097 uniform points.
 constexpr int kSortOne = 4096;
 
 __global__ void k_bounds_init(int *b, int num_clouds)
