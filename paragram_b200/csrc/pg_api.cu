@@ -432,7 +432,7 @@ static int build_impl(int64_t n, int num_clouds, const int32_t *cloud_offsets, c
     const int64_t cells = ranged ? range_end - range_begin : n;
     cl.lanes = cells >= kLaneMinCells && num_clouds == 1 && leaf <= kDefaultLeaf && !cl.fp32_only &&
                !opt.radius_out && !opt.work_out && opt.blocks_per_sm != 3;
-    cl.choice = LaneChoice{ws.counters, 1, cells < (guesses ? kLaneAnyCellsGuess : kLaneAnyCells)};
+    cl.choice = LaneChoice{ws.counters, 1, !guesses && cells < kLaneAnyCells};
     if (cl.lanes)
         cl.choice.groups = lane_survey_launch(ws, n, st);
     int chunks = sync ? plan_chunks(n, opt.num_chunks) : std::max(opt.num_chunks, 1);

@@ -67,18 +67,18 @@ constexpr uint32_t kBigFlag = 0x40000000u; // deg[] flag: row lives in the defer
 // Levels: in a build that the pass finishes in one or two waves, cells beside a far denser region are listed, and
 // the pass over the list takes as long as the slowest of them. Variance of the levels 2 to 3 in uniform points
 // (warp-per-cell pass 2.28 ms, cell-per-lane 2.11 at 40,000), 4.2 in 64 Gaussians of similar widths (2.18, 2.20),
-// 4.9 in 500 narrow ones (2.47, 3.03), 14 to 21 with widths from 0.005 to 0.1 (2.50, 2.80 at 40,000; 3.09, 3.14 at
-// 56,000; 3.24, 3.27 at 60,000; 4.02, 3.70 at 80,000; with the previous step's diagram as guesses 2.36, 2.39 at
-// 36,000; 2.91, 2.87 at 48,000; 3.24, 3.03 at 56,000).
+// 4.9 in 500 narrow ones (2.47, 3.03), 14 to 21 with widths from 0.005 to 0.1 (five clouds each, means: 2.57, 2.83
+// at 44,000; 3.07, 3.07 at 56,000; 3.39, 3.18 at 64,000). With initial guesses the pass is as fast or faster from the
+// start (2.19, 2.16 at 33,000; 2.89, 2.79 at 48,000).
 constexpr int kSurveyGroups = 512;
 constexpr int kLaneFlatShare = 10;         // declined above one flat group in ten
 constexpr int kLaneLevelVar2 = 9;          // declined below kLaneAnyCells above half this variance of the levels
-constexpr int64_t kLaneAnyCells = 60000, kLaneAnyCellsGuess = 46000; // (the latter with initial guesses)
+constexpr int64_t kLaneAnyCells = 56000;
 struct LaneChoice
 {
     const int *counters; // the workspace's
     int groups;          // groups sampled
-    int few;             // the build has fewer than kLaneAnyCells(Guess) cells
+    int few;             // the build has fewer than kLaneAnyCells cells and no initial guesses
 
     __host__ __device__ bool declined() const
     {

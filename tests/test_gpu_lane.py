@@ -84,6 +84,7 @@ def test_lane_pass_equals_oracle(dev, oracle, kind, n):
 
 @pytest.mark.parametrize("kind,n,taken", [("uniform", MIN - 1, False), ("uniform", MIN, True), ("heavy", 40_000, True),
                                           ("lattice", 35_937, True), ("clustered", MIN + 5, False),
+                                          ("clustered", 55_999, False), ("clustered", 56_000, True),
                                           ("clustered", 60_001, True), ("surface", 36_001, False),
                                           ("surface", 100_000, False), ("surface", 400_000, True)])
 def test_lane_pass_choice(dev, kind, n, taken):
